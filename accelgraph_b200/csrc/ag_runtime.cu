@@ -28,6 +28,7 @@
 
 #include "ag_device.h"
 #include "ag_internal.h"
+#include "ag_solve.h"
 
 /* ------------------------------------------------------------ context */
 struct AgContext
@@ -370,6 +371,13 @@ struct ag_graph_s
     AgControl *ctl;
     float *init_buf;
     uint32_t *flag;
+    /* the solve kernel's bins and its hub rows' state; none (sync NULL) on a
+     * graph that the pull kernel's loop runs */
+    AgBinPlan bin;
+    double *hub_sum;
+    uint32_t *hub_words, *hub_seen;
+    uint8_t *hub_pred8;
+    uint32_t *sync;
     AgExec exe[3][2];
     int have_exe[3][2];
     /* data-driven mode: its launch graphs (FAST, EXACT) */
@@ -502,6 +510,18 @@ extern "C" ag_status_t ag_graph_release(ag_graph_t g)
     dev_free(g->hub_vals);
     dev_free(g->hub_pred);
     dev_free(g->hub_t);
+    dev_free(g->bin.bins);
+    dev_free(g->bin.hubs);
+    dev_free(g->bin.brow);
+    dev_free(g->bin.ubase);
+    dev_free(g->bin.ids);
+    dev_free(g->bin.pre);
+    dev_free(g->bin.tmp);
+    dev_free(g->hub_sum);
+    dev_free(g->hub_words);
+    dev_free(g->hub_seen);
+    dev_free(g->hub_pred8);
+    dev_free(g->sync);
     dev_free(g->ctl);
     dev_free(g->init_buf);
     dev_free(g->flag);
@@ -604,6 +624,66 @@ static ag_status_t plan_device(ag_graph_s *g, uint32_t cap, uint32_t whub)
     g->ntasks_exact = ne;
     g->nparts = tot[0];
     g->num_hub_rows = tot[3];
+    return AG_OK;
+}
+
+/* Graphs of more in-edges run on the pull kernel's loop: there the solve
+ * kernel's bins wait longer for their gathers than the pull kernel's warps,
+ * which overlap theirs item by item.  us per pass, pull kernel / solve kernel
+ * (EXACT; R-MAT, 16 edges per vertex): 54 / 21 at 1 M in-edges, 127 / 83 at
+ * 16 M, 130 / 91 at 18 M, but 336 / 348 at 65 M; FAST order 20 / 13, 65.8 /
+ * 66.4, 81 / 79, 218 / 295. */
+#ifndef AG_BIN_MAX_EDGES
+#define AG_BIN_MAX_EDGES 20000000u
+#endif
+/* Row weight per bin: one bin for every group of the persistent grid on a
+ * small graph, several of at most AG_BIN_QUANTUM on a larger one (the same
+ * number for each group).  A larger bin has fewer waits, a smaller one leaves
+ * more of the SM's memory to L1: us per pass (FAST / EXACT) at 16 M in-edges
+ * 94 / 104 with 4096, 71 / 84 with 8192, 66 / 83 with 12288, 85 / 101 with
+ * 16384. */
+#ifndef AG_BIN_QUANTUM
+#define AG_BIN_QUANTUM 12288u
+#endif
+static uint32_t bin_quantum(uint64_t weight)
+{
+    const uint32_t qmax = AG_BIN_QUANTUM;
+    const uint64_t groups = (uint64_t)std::max(1, g_ctx.num_sms) * AG_SUBS;
+    const uint64_t waves = (weight + groups * qmax - 1) / (groups * qmax);
+    const uint64_t q = waves ? (weight + groups * waves - 1) / (groups * waves) : 1;
+    return (uint32_t)std::max<uint64_t>(512, std::min<uint64_t>(q, qmax));
+}
+
+/* the solve kernel's bins, from the device row offsets and their totals
+ * (ag_bins_count, already waited for) */
+static ag_status_t plan_bins(ag_graph_s *g, uint64_t total)
+{
+    cudaStream_t s = g_ctx.stream;
+    AgBinPlan *b = &g->bin;
+    ag_status_t st = AG_OK;
+    ag_bins_shape(b, total, bin_quantum((total & ((1ull << 40) - 1)) + (total >> 40) * AG_BIN_HUB), g->ngraphs);
+    const size_t words = ag_bins_brow_words(b, g->N);
+    b->bins = (AgBin *)dev_alloc(g, (size_t)b->nbins * sizeof(AgBin), &st);
+    b->hubs = (uint4 *)dev_alloc(g, (size_t)b->nhub * sizeof(uint4), &st);
+    b->brow = (uint32_t *)dev_alloc(g, words * 4, &st);
+    b->ubase = (uint32_t *)dev_alloc(g, words / 32 * 4 + 16, &st);
+    b->ids = (uint32_t *)dev_alloc(g, (size_t)b->nslots * 4, &st);
+    g->hub_sum = (double *)dev_alloc(g, (size_t)b->nhub * 8, &st);
+    g->hub_words = (uint32_t *)dev_alloc(g, (size_t)b->nhub * AG_BIN_ROUNDS * 4, &st);
+    g->hub_seen = (uint32_t *)dev_alloc(g, (size_t)b->nhub * 4, &st);
+    g->hub_pred8 = (uint8_t *)dev_alloc(g, (size_t)b->nhub * AG_BIN_ROUNDS, &st);
+    g->sync = (uint32_t *)dev_alloc(g, AG_SYNC_WORDS * 4, &st);
+    if (st != AG_OK)
+        return st;
+    cudaError_t e = ag_bins_rows(g->row_off, g->N, g->gstart, g->ngraphs, b, s);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(g->hub_seen, 0, (size_t)b->nhub * 4 + (b->nhub ? 0 : 16), s);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(g->sync, 0, AG_SYNC_WORDS * 4, s);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return ag_set_error(AG_ERR_CUDA, "bin planning failed: %s", cudaGetErrorString(e));
+    }
     return AG_OK;
 }
 
@@ -886,7 +966,14 @@ static ag_status_t upload_impl(const struct GraphCSR *graph, uint32_t flags, con
             UPFAIL(st);
         UP(cudaMemcpyAsync(g->gstart, gstart_host, (size_t)(ngraphs + 1) * 4, cudaMemcpyHostToDevice, s));
     }
+    /* a row partition runs pass by pass on the pull kernel, without bins */
+    const bool bins = gather_n == 0 && E <= AG_BIN_MAX_EDGES;
+    uint64_t bin_total = 0;
+    if (bins)
+        UP(ag_bins_count(g->row_off, N, &g->bin, &bin_total, s));
     st = plan_device(g, g->tiles.task_edges, g->tiles.hub_chunk);
+    if (st == AG_OK && bins)
+        st = plan_bins(g, bin_total);
     if (st != AG_OK)
         UPFAIL(st);
 
@@ -921,6 +1008,13 @@ static ag_status_t upload_impl(const struct GraphCSR *graph, uint32_t flags, con
         g->device_bytes -= (uint64_t)(N + 1) * 4 + (uint64_t)g->E4 * 4 * (want_w ? 2 : 1) + (uint64_t)N * 4 + 16;
         off_old = ids_old = outdeg_old = nullptr;
         w_old = nullptr;
+    }
+    if (bins) {
+        UP(ag_bins_ids(g->row_off, g->ids, &g->bin, s));
+        dev_free(g->bin.pre);
+        dev_free(g->bin.tmp);
+        g->bin.pre = nullptr;
+        g->bin.tmp = nullptr;
     }
     UP(cudaEventCreate(&g->ev0));
     UP(cudaEventCreate(&g->ev1));
@@ -1099,6 +1193,67 @@ static const void *solve_pull_kernel(const ag_graph_s *g, int prec, int exact, i
 static size_t solve_smem(const ag_graph_s *g, int prec)
 {
     return is_int_prec(prec) ? ag_fixed_smem_bytes(int_bytes(prec)) : pull_smem(g);
+}
+
+/* polls of a grid barrier of the solve kernel before it gives up (each a
+ * round trip to L2: tens of seconds, far above the longest pass) */
+#define AG_GRID_SPINS (1u << 26)
+
+/* a solve, or parts of one, as cooperative launches of the solve kernel: one
+ * CTA on every SM (fewer on a graph of fewer bins) */
+static ag_status_t solve_launch(ag_graph_s *g, int prec, int exact, int dd, const AgRunConfig &run)
+{
+    cudaStream_t s = g_ctx.stream;
+    AgSolveParams q;
+    memset(&q, 0, sizeof(q));
+    q.p = base_params(g, exact);
+    q.bins = g->bin.bins;
+    q.hubs = g->bin.hubs;
+    q.brow = g->bin.brow;
+    q.ubase = g->bin.ubase;
+    q.ids = g->bin.ids;
+    q.nbins = g->bin.nbins;
+    q.nhub = g->bin.nhub;
+    q.buf = g->bin.buf;
+    q.per_bin = std::min<uint32_t>(16, std::max<uint32_t>(1, q.buf / AG_BIN_HUB));
+    q.nhb = (q.nhub + q.per_bin - 1) / q.per_bin;
+    q.hub_sum = g->hub_sum;
+    q.hub_words = g->hub_words;
+    q.hub_pred = g->hub_pred8;
+    q.hub_seen = g->hub_seen;
+    q.sync = g->sync;
+    q.spins = AG_GRID_SPINS;
+    const size_t bufs = (size_t)AG_SUBS * q.buf * 4;
+    const uint32_t fit = (uint32_t)((AG_SMEM_MAX - AG_SMEM_STATIC - bufs) / 4) & ~63u;
+    q.p.hot_n = std::min(q.p.hot_n, fit);
+    q.p.hot_n16 = std::min<uint32_t>(2 * q.p.hot_n, g->N & ~63u);
+    const size_t smem = (size_t)q.p.hot_n * 4 + bufs;
+    const void *k = ag_solve_kernel_ptr(dd ? AG_MODE_DD : g->ngraphs ? AG_MODE_MULTI : AG_MODE_PR, prec, exact);
+    ag_status_t st = pull_kernel_prepare(k, smem);
+    if (st != AG_OK)
+        return st;
+    const unsigned grid = (unsigned)std::max<uint64_t>(
+        1, std::min<uint64_t>((uint64_t)g_ctx.num_sms, (uint64_t)q.nhb + q.nbins));
+    AgRunConfig r = run;
+    void *args[2] = {&q, &r};
+    const char *mode = getenv("AG_LAUNCH_MODE");
+    if (mode && strcmp(mode, "stream") == 0) {
+        /* profiling form: one launch per part (a profiler sees every pass);
+         * passes after the loop has ended return at once */
+        q.do_init = 1;
+        AG_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(AG_SOLVE_BLK), args, smem, s));
+        q.do_init = 0;
+        q.max_pass = 1;
+        for (uint32_t i = 0; i < run.max_iter; ++i)
+            AG_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(AG_SOLVE_BLK), args, smem, s));
+        q.max_pass = 0;
+        q.do_norm = 1;
+    } else {
+        q.do_init = q.do_norm = 1;
+        q.max_pass = 0xFFFFFFFFu;
+    }
+    AG_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(AG_SOLVE_BLK), args, smem, s));
+    return AG_OK;
 }
 
 static dim3 elem_grid(const ag_graph_s *g)
@@ -1629,12 +1784,12 @@ extern "C" ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations,
         /* rebuild cached graphs: their parameters carry the warm-start pointer */
         drop_execs(g);
     }
-    if (!have_exec(g, prec, exact, dd)) {
+    const bool bins = !ip && g->sync;
+    if (!bins && !have_exec(g, prec, exact, dd)) {
         st = build_exec(g, prec, exact, dd);
         if (st != AG_OK)
             return st;
     }
-    AgExec *x = exec_slot(g, prec, exact, dd);
     cudaStream_t s = g_ctx.stream;
     if (o.init_ranks && g->N)
         AG_CUDA(cudaMemcpyAsync(g->init_buf, o.init_ranks, (size_t)g->N * 4,
@@ -1645,6 +1800,18 @@ extern "C" ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations,
     run.use_init = o.init_ranks ? 1u : 0u;
     run.eps = epsilon;
     run.switch_residual = o.switch_residual > 0 ? o.switch_residual : 1e-4;
+    if (bins) {
+        AG_CUDA(cudaEventRecord(g->ev0, s));
+        st = solve_launch(g, prec, exact, dd, run);
+        if (st != AG_OK)
+            return st;
+        AG_CUDA(cudaEventRecord(g->ev1, s));
+        g->launched = 1;
+        g->last_prec = prec;
+        g->last_exact = exact;
+        return AG_OK;
+    }
+    AgExec *x = exec_slot(g, prec, exact, dd);
     void *init_args[2] = {&x->params, &run};
     cudaKernelNodeParams kp;
     AG_CUDA(cudaGraphKernelNodeGetParams(x->init_node, &kp));
@@ -1737,6 +1904,12 @@ extern "C" ag_status_t ag_pagerank_fetch(ag_graph_t g, float *ranks, ag_pr_resul
     }
     const uint32_t fault = hc->fault;
     free(hc);
+    if (fault & 2u) {
+        /* the solve gave up part way: the next one starts with a fresh barrier */
+        AG_CUDA(cudaMemset(g->sync, 0, AG_SYNC_WORDS * 4));
+        return ag_set_error(AG_ERR_DEVICE_WAIT, "a grid barrier of the solve kernel ran out before every CTA arrived; "
+                            "the solve did not finish");
+    }
     if (fault)
         return ag_set_error(AG_ERR_DEVICE_WAIT, "a pull kernel's bounded wait for its hot-table copy ran out "
                             "(the copies completed before the kernel went on; results are filled in)");

@@ -1,0 +1,52 @@
+/*
+ * ag_solve.h -- parameters of the solve kernel (ag_solve.cu).
+ */
+#ifndef AG_SOLVE_H
+#define AG_SOLVE_H
+
+#include "ag_bins.h"
+#include "ag_device.h"
+
+#ifndef AG_SUBS
+#define AG_SUBS 2             /* warp groups of a CTA, each on its own bin      */
+#endif
+#define AG_SOLVE_BLK 1024
+#define AG_SUB_THREADS (AG_SOLVE_BLK / AG_SUBS)
+#define AG_SUB_WARPS (AG_SUB_THREADS / 32)
+
+/* words of AgSolveParams::sync */
+#define AG_SYNC_COUNT 0       /* CTAs that have arrived                         */
+#define AG_SYNC_GEN 1         /* barriers passed << 3 | flags                   */
+#define AG_SYNC_BIN 2         /* bins handed out in this pass                   */
+#define AG_SYNC_WORDS 4
+#define AG_GEN_STOP 1u
+#define AG_GEN_READ_LOW 2u
+#define AG_GEN_WRITE_LOW 4u
+
+typedef struct AgSolveParams
+{
+    AgPullParams p;
+    const AgBin *bins;
+    const uint4 *hubs;
+    const uint32_t *brow, *ubase, *ids;
+    uint32_t nbins, nhub;     /* row bins, hub chunks                           */
+    uint32_t per_bin, nhb;    /* hub chunks per bin, bins they make             */
+    uint32_t buf;             /* floats of a group's buffer                     */
+    double *hub_sum;          /* per chunk: FAST partial sum, EXACT head sum    */
+    uint32_t *hub_words;      /* EXACT: AG_BIN_ROUNDS words per chunk           */
+    uint8_t *hub_pred;        /* EXACT: biased exponent at each round's start   */
+    uint32_t *hub_seen;       /* per chunk (used at a row's first): chunks done */
+    uint32_t *sync;           /* AG_SYNC_WORDS                                  */
+    uint32_t spins;           /* polls of a grid barrier before it gives up     */
+    uint32_t do_init, do_norm, max_pass; /* parts of a solve in this launch     */
+} AgSolveParams;
+
+#ifdef __cplusplus
+extern "C" {
+#endif
+const void *ag_solve_kernel_ptr(int mode, int prec, int exact);
+#ifdef __cplusplus
+}
+#endif
+
+#endif /* AG_SOLVE_H */
