@@ -122,7 +122,7 @@ static inline unsigned ag_sm_grid(unsigned per_sm)
 #define AG_MODE_SPMV 1
 #define AG_MODE_MULTI 2   /* PageRank over a union of independent graphs,
                              each with its own convergence                  */
-#define AG_MODE_DD 3      /* data-driven PageRank: a rank is replaced only
+#define AG_MODE_DD 3      /* solve kernel: data-driven PageRank, a rank is replaced only
                              when it moves by at least epsilon, and only rows
                              with a changed in-neighbour (or the first pass)
                              are updated; a change is signalled by the sign
@@ -324,9 +324,9 @@ cudaError_t ag_set_u32(uint32_t *p, uint32_t v, cudaStream_t s);
 struct ag_graph_s;
 int32_t ag_rt_graph_view(struct ag_graph_s *g, AgGraphView *v);
 
-/* Kernel selection (prec: 0 fp32, 1 bf16, 2 fp16; exact: stream-order sums) */
-const void *ag_pull_kernel_ptr(int mode, int prec, int exact);
-const void *ag_init_kernel_ptr(int prec);
+/* Kernel selection (exact: stream-order sums) */
+const void *ag_pull_kernel_ptr(int mode, int exact);
+const void *ag_init_kernel_ptr(void);
 const void *ag_normalize_kernel_ptr(void);
 /* integer pulls: contributions of `bytes` (8, 4, 2, 1) bytes, fixed point or
  * quantised; gather = 1: only the integer sums.  Their init kernel, the

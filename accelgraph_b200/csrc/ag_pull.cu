@@ -1,5 +1,7 @@
 /*
- * ag_pull.cu -- sm_100a kernels of the pull PageRank / SpMV hot path.
+ * ag_pull.cu -- sm_100a pass-by-pass kernels of the pull: the SpMV product, a
+ * row partition's pass, and the passes of a large union of graphs.  Whole
+ * solves run on the solve kernel (ag_solve.cu).
  *
  * One pull pass (reference: the host contribution loop pageRank.c:1026-1033,
  * the accelerator gather of the cu_PageRank CSR PULL compute units, whose arithmetic the RTL
@@ -37,8 +39,6 @@
  * chunk to arrive adds them in stream order.
  * All reductions have a fixed order: results do not depend on scheduling.
  */
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -95,23 +95,6 @@ __device__ __forceinline__ bool ag_mbar_wait(uint64_t *bar, uint32_t phase, uint
     return false;
 }
 
-/* 16-bit contribution formats of the precision form */
-template <int PREC>
-__device__ __forceinline__ float ag_low_to_f32(uint16_t h)
-{
-    if (PREC == 1)
-        return __uint_as_float(((uint32_t)h) << 16);
-    return __half2float(__ushort_as_half(h));
-}
-
-template <int PREC>
-__device__ __forceinline__ uint16_t ag_f32_to_low(float f)
-{
-    if (PREC == 1)
-        return __bfloat16_as_ushort(__float2bfloat16_rn(f));
-    return __half_as_ushort(__float2half_rn(f));
-}
-
 /* ----------------------------------------------------- reductions */
 __device__ __forceinline__ float ag_warp_sum_f(float v)
 {
@@ -138,69 +121,41 @@ __device__ __forceinline__ uint32_t ag_warp_sum_u(uint32_t v)
 }
 
 /* ------------------------------------------------------------- kernel */
-template <int MODE, int PREC, bool EXACT, bool LOW = false>
+template <int MODE, bool EXACT>
 struct AgPass
 {
     const AgPullParams &p;
     uint64_t pol_first, pol_last;
     const float *c_in32;
-    const uint16_t *c_in16;
     float *c_out32;
-    uint16_t *c_out16;
-    /* this pass reads 16-bit contributions (fixed per kernel body, so that
-     * the 16-bit and 32-bit passes each get their own loads and registers) */
-    static constexpr bool read_low = PREC != 0 && LOW;
-    uint32_t write_low;
     double eps;
     double my_err;
     uint32_t my_active;
     const float *hot32;     /* shared-memory copy of the first hot_n values */
-    const uint16_t *hot16;
     uint32_t hot_n;
-    bool dd_all;              /* data-driven mode: the first pass, where every row is active */
 
     __device__ __forceinline__ AgPass(const AgPullParams &pp) : p(pp)
     {
         hot32 = nullptr;
-        hot16 = nullptr;
         hot_n = 0;
         pol_first = ag_policy_evict_first();
         pol_last = ag_policy_evict_last();
         my_err = 0.0;
         my_active = 0;
-        write_low = 0;
         eps = 0.0;
         c_in32 = nullptr;
-        c_in16 = nullptr;
         c_out32 = nullptr;
-        c_out16 = nullptr;
-        dd_all = false;
         if (MODE != AG_MODE_SPMV) {
             const uint32_t pass = p.ctl->iter;
             eps = p.ctl->eps;
-            if (PREC != 0)
-                write_low = p.ctl->mode_write;
             const bool odd = (pass & 1u) != 0;
             c_in32 = odd ? p.c32_1 : p.c32_0;
             c_out32 = odd ? p.c32_0 : p.c32_1;
-            c_in16 = odd ? p.c16_1 : p.c16_0;
-            c_out16 = odd ? p.c16_0 : p.c16_1;
-            if (MODE == AG_MODE_DD)
-                dd_all = pass == 0;
         }
     }
 
-    /* the vector this pass gathers from, and its element size */
-    __device__ __forceinline__ const void *gather_source() const
-    {
-        if (MODE == AG_MODE_SPMV)
-            return p.x;
-        if (PREC != 0 && read_low)
-            return c_in16;
-        return c_in32;
-    }
-
-    __device__ __forceinline__ uint32_t gather_elem_bytes() const { return (PREC != 0 && read_low) ? 2u : 4u; }
+    /* the vector this pass gathers from */
+    __device__ __forceinline__ const void *gather_source() const { return MODE == AG_MODE_SPMV ? p.x : c_in32; }
 
     /* value gathered for an in-edge with source u (weight wj for SpMV):
      * from the shared-memory table when u is hot, else from global memory */
@@ -213,10 +168,6 @@ struct AgPass
                 return xv;
             return __fmul_rn(wj, xv);
         }
-        if (PREC != 0 && read_low)
-            return ag_low_to_f32<PREC>((u < hot_n) ? hot16[u]
-                                       : (u < p.warm_n ? ag_ld_gather_u16(c_in16 + u, pol_last)
-                                                       : ag_ld_cold_u16(c_in16 + u, pol_last)));
         return (u < hot_n) ? hot32[u]
                            : (u < p.warm_n ? ag_ld_gather_f32(c_in32 + u, pol_last) : ag_ld_cold_f32(c_in32 + u, pol_last));
     }
@@ -235,40 +186,7 @@ struct AgPass
         my_err += err;
         my_active += (err >= eps) ? 1u : 0u;
         const float c = od ? __fdiv_rn(rn, __uint2float_rn(od)) : 0.0f;
-        if (PREC != 0 && write_low)
-            ag_st_keep_u16(c_out16 + r, ag_f32_to_low<PREC>(c), pol_last);
-        else
-            ag_st_keep_f32(c_out32 + p.c_base + r, c, pol_last);
-    }
-
-    /* Data-driven mode (the reference's worklist pull, pageRank.c:2810-2969).
-     * A row is on the worklist of a pass when the pass is the first or one of
-     * its in-neighbours changed in the pass before.  A vertex that changes
-     * writes its next contribution with the sign bit set (contributions are
-     * otherwise never negative), so a row learns that from the values it
-     * gathers anyway: it sums their magnitudes, which are the reference's
-     * contributions bit for bit, and ORs their sign bits.  Nothing is
-     * scattered to out-neighbours. */
-    static __device__ __forceinline__ uint32_t dd_neg(float v) { return __float_as_uint(v) >> 31; }
-
-    /* the update of a row (pageRank.c:2896-2916): rows off the worklist and
-     * rows that moved by less than epsilon keep rank and contribution (sign
-     * cleared); an active row's residual always counts */
-    __device__ __forceinline__ void finish_dd(uint32_t r, float s, float rp, uint32_t od, bool act)
-    {
-        if (act) {
-            const float rn = __fadd_rn(p.base, __fmul_rn(p.damp, s));
-            const double err = (double)fabsf(__fsub_rn(rn, rp));
-            my_err += err;
-            if (err >= eps) {
-                p.rank[r] = rn;
-                const float c = od ? __fdiv_rn(rn, __uint2float_rn(od)) : 0.0f;
-                ag_st_keep_f32(c_out32 + r, __uint_as_float(__float_as_uint(c) | 0x80000000u), pol_last);
-                ++my_active;
-                return;
-            }
-        }
-        ag_st_keep_f32(c_out32 + r, fabsf(__ldg(c_in32 + r)), pol_last);
+        ag_st_keep_f32(c_out32 + p.c_base + r, c, pol_last);
     }
 
     /* two 16-byte groups of in-edges per lane: quads qa and qa + 32 (ids and,
@@ -386,7 +304,7 @@ struct AgPass
      * the next pair is in flight while the current one is gathered and
      * added (fixed lane assignment, edge order within a lane) */
     __device__ __forceinline__ float strided_partial(uint32_t eb, uint32_t ee, uint32_t lane,
-                                                     const Pair &first, uint32_t &neg) const
+                                                     const Pair &first) const
     {
         /* two rounds of gathers in flight: the values of round k are added
          * while those of round k + 1 travel and the ids of round k + 2 load.
@@ -425,12 +343,7 @@ struct AgPass
             gather8(nxt, qn, eb, ee, vn, in);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                if (MODE == AG_MODE_DD) {
-                    neg |= dd_neg(v[k]);
-                    s = __fadd_rn(s, fabsf(v[k]));
-                } else {
-                    s = __fadd_rn(s, v[k]);
-                }
+                s = __fadd_rn(s, v[k]);
                 v[k] = vn[k];
             }
             nxt = nn;
@@ -495,8 +408,7 @@ struct AgPass
      *    (no partial sum can leave the binade: the steps are >= 0).
      *    Otherwise the round's staged values are added one by one.  It then
      *    records where each chunk began, for the next pass.
-     * Data-driven passes stage the values with their sign tags and sum the
-     * magnitudes. */
+     */
 
     /* s rebuilt from its exponent bits and M (M in [2^23, 2^24)) */
     static __device__ __forceinline__ float exact_make(uint32_t ex, uint32_t m)
@@ -523,7 +435,7 @@ struct AgPass
     static __device__ __forceinline__ bool hub_staged(uint32_t pr)
     {
         const uint32_t e = pr & 0xffu;
-        return MODE == AG_MODE_SPMV || PREC != 0 || e < 24u || e > 253u || (pr & AG_XFELL) != 0u;
+        return MODE == AG_MODE_SPMV || e < 24u || e > 253u || (pr & AG_XFELL) != 0u;
     }
 
     /* EXACT-order hub chunk after the first: stages (when `stage`) the
@@ -531,14 +443,13 @@ struct AgPass
      * dst[j - o0], and writes
      * per round the totals of its integer steps at binade e and e + 1
      * (words[2k], words[2k+1]; AG_XNOT when they do not apply or e is
-     * unknown) and the chunk's sign tag (words[AG_XWORDS - 1]). */
+     * unknown). */
     __device__ __forceinline__ void hub_steps(float *dst, uint32_t o0, uint32_t eb, uint32_t ee, uint32_t lane,
                                               const Pair &first, uint32_t e, bool stage, uint32_t *words) const
     {
         const uint32_t q1 = (ee + 3u) >> 2;
         const bool known = (e >= 24u) & (e <= 253u);
         const float sc = known ? exact_scale(e) : 0.0f;
-        uint32_t neg = 0;
         /* round k's values v (quads qa and qa + 32): staged when asked, and
          * their integer steps summed.  Values outside [eb, ee) gather as +0,
          * whose step is 0. */
@@ -559,12 +470,7 @@ struct AgPass
                 bool b0 = false, b1 = false;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    float x = v[i];
-                    if (MODE == AG_MODE_DD) {
-                        neg |= dd_neg(x);
-                        x = fabsf(x);
-                    }
-                    const float x0 = __fmul_rn(x, sc);
+                    const float x0 = __fmul_rn(v[i], sc);
                     /* one binade up: half the units (exact, or a value far
                      * below one unit either way) */
                     const float x1 = __fmul_rn(x0, 0.5f);
@@ -580,10 +486,6 @@ struct AgPass
                     words[2 * k] = b0 ? AG_XNOT : t0;
                     words[2 * k + 1] = b1 ? AG_XNOT : t1;
                 }
-            } else if (MODE == AG_MODE_DD) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    neg |= dd_neg(v[i]);
             }
         };
         /* the loop runs on the round's first quad, the same in every lane:
@@ -629,11 +531,6 @@ struct AgPass
         }
         if (!known && lane < AG_XROUNDS)
             words[2 * lane] = words[2 * lane + 1] = AG_XNOT;
-        if (MODE == AG_MODE_DD) {
-            neg = __any_sync(0xffffffffu, neg) ? 1u : 0u;
-            if (lane == 0)
-                words[AG_XWORDS - 1] = neg;
-        }
     }
 
     /* EXACT-order hub row, on the warp of its last chunk to arrive: the
@@ -642,26 +539,15 @@ struct AgPass
      * chunks' round totals and, where a total does not apply, the staged
      * values (row_vals[j - o0]) added one by one through the warp's
      * shared-memory slice.  Records each chunk's starting binade for the
-     * next pass.  Data-driven passes OR the sign tags into `neg`. */
-    struct XSum
-    {
-        float s;
-        uint32_t neg;
-    };
-
+     * next pass. */
     /* static, with plain arguments: a call of a member would need the
      * kernel's parameter block in local memory */
-    static __device__ __noinline__ XSum hub_compose(const uint32_t *hub_part, const uint32_t *hub_t,
+    static __device__ __noinline__ float hub_compose(const uint32_t *hub_part, const uint32_t *hub_t,
                                                     uint32_t *hub_pred, const float *row_vals, const uint32_t *ids,
                                                     const float *c_in, float *vals, uint32_t whub, uint32_t o0,
                                                     uint32_t deg, uint32_t pbase, uint32_t nch, uint32_t lane)
     {
-        uint32_t neg = 0;
         float s = __uint_as_float(__ldcg(hub_part + pbase));
-        if (MODE == AG_MODE_DD) {
-            neg |= dd_neg(s);
-            s = fabsf(s);
-        }
         const uint32_t *wp = hub_t + (size_t)(pbase + 1) * AG_XWORDS;
         uint32_t wa = __ldcg(wp + lane), wb = __ldcg(wp + 32 + lane);
         uint32_t pr = __ldcg(hub_pred + pbase + 1);
@@ -674,8 +560,6 @@ struct AgPass
                 nb = __ldcg(wn + 32 + lane);
                 npr = __ldcg(hub_pred + pbase + c + 1);
             }
-            if (MODE == AG_MODE_DD)
-                neg |= __shfl_sync(0xffffffffu, wb, 31) & 1u;
             const uint32_t e = pr & 0xffu;
             const uint32_t e_start = __float_as_uint(s) >> 23;
             bool fell = false;
@@ -718,7 +602,7 @@ struct AgPass
                     }
                     __syncwarp();
                     if (lane == 0)
-                        s = seq_sum(vals, 0, hi - lo, s, false, neg);
+                        s = seq_sum(vals, 0, hi - lo, s, false);
                     s = __shfl_sync(0xffffffffu, s, 0);
                     fell = true;
                 }
@@ -729,45 +613,36 @@ struct AgPass
             wb = nb;
             pr = npr;
         }
-        return XSum{s, neg};
+        return s;
     }
 
     /* the stream-order sum of vals[a, b) (the warp's shared-memory slice)
      * by the calling lane alone, continuing s, or starting with vals[a] when
      * `first`: four values per 16-byte shared load once the index is
-     * aligned, one binary32 add after another.  Data-driven passes add the
-     * magnitudes and OR the sign tags into `neg`. */
-    static __device__ __forceinline__ float seq_sum(const float *vals, uint32_t a, uint32_t b, float s, bool first,
-                                                    uint32_t &neg)
+     * aligned, one binary32 add after another. */
+    static __device__ __forceinline__ float seq_sum(const float *vals, uint32_t a, uint32_t b, float s, bool first)
     {
-        auto val = [&](float v) {
-            if (MODE == AG_MODE_DD) {
-                neg |= dd_neg(v);
-                v = fabsf(v);
-            }
-            return v;
-        };
         uint32_t j = a;
         if (first && j < b) {
-            s = val(vals[j]);
+            s = vals[j];
             ++j;
         }
         for (; j < b && (j & 3u); ++j)
-            s = __fadd_rn(s, val(vals[j]));
+            s = __fadd_rn(s, vals[j]);
         for (; j + 8u <= b; j += 8u) {
             const float4 q0 = reinterpret_cast<const float4 *>(vals)[j >> 2];
             const float4 q1 = reinterpret_cast<const float4 *>(vals)[(j >> 2) + 1];
-            s = __fadd_rn(s, val(q0.x));
-            s = __fadd_rn(s, val(q0.y));
-            s = __fadd_rn(s, val(q0.z));
-            s = __fadd_rn(s, val(q0.w));
-            s = __fadd_rn(s, val(q1.x));
-            s = __fadd_rn(s, val(q1.y));
-            s = __fadd_rn(s, val(q1.z));
-            s = __fadd_rn(s, val(q1.w));
+            s = __fadd_rn(s, q0.x);
+            s = __fadd_rn(s, q0.y);
+            s = __fadd_rn(s, q0.z);
+            s = __fadd_rn(s, q0.w);
+            s = __fadd_rn(s, q1.x);
+            s = __fadd_rn(s, q1.y);
+            s = __fadd_rn(s, q1.z);
+            s = __fadd_rn(s, q1.w);
         }
         for (; j < b; ++j)
-            s = __fadd_rn(s, val(vals[j]));
+            s = __fadd_rn(s, vals[j]);
         return s;
     }
 
@@ -781,7 +656,7 @@ struct AgPass
      * lane's chain costs about 1.25 instructions per value.  `first` is the
      * range's first id pair; the sum is lane 0's. */
     __device__ __forceinline__ float ordered_sum(float *vals, uint32_t eb, uint32_t ee, uint32_t lane,
-                                                 const Pair &first, uint32_t &neg) const
+                                                 const Pair &first) const
     {
         uint32_t cb = eb, ce = min(ee, (eb & ~3u) + (uint32_t)AG_WCAP);
         /* the ids of a round are requested one round before its gathers */
@@ -793,7 +668,7 @@ struct AgPass
             const uint32_t nb = ce, ne = min(ee, ce + (uint32_t)AG_WCAP);
             if (nb >= ee) {
                 if (lane == 0)
-                    s = seq_sum(vals, 0, ce - cb, s, cb == eb, neg);
+                    s = seq_sum(vals, 0, ce - cb, s, cb == eb);
                 return s;
             }
             /* the next round's gathers travel while this one is added */
@@ -801,7 +676,7 @@ struct AgPass
             stage_issue(ids, nb, ne, lane, w);
             ids = prefetch(ne, min(ee, ne + (uint32_t)AG_WCAP), lane);
             if (lane == 0)
-                s = seq_sum(vals, 0, ce - cb, s, cb == eb, neg);
+                s = seq_sum(vals, 0, ce - cb, s, cb == eb);
             __syncwarp();
             stage_commit(vals, nb, ne, lane, w);
             cb = nb;
@@ -863,12 +738,12 @@ static __device__ __forceinline__ uint32_t ag_steal_next(uint32_t *steal, AgStea
     return ntasks;
 }
 
-/* one pull pass on this CTA; LOW: the pass reads 16-bit contributions */
-template <int MODE, int PREC, bool EXACT, bool LOW>
+/* one pull pass on this CTA */
+template <int MODE, bool EXACT>
 __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_redd, uint32_t *s_redu,
                                              uint32_t &s_last, uint64_t &s_bar)
 {
-    AgPass<MODE, PREC, EXACT, LOW> ps(p);
+    AgPass<MODE, EXACT> ps(p);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float *vals = reinterpret_cast<float *>(ag_dsmem) + warp * AG_WCAP;
     unsigned char *hot = ag_dsmem + AG_STAGE_BYTES;
@@ -878,9 +753,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
      * copy per 32 KB, completing on an mbarrier that every thread waits on
      * (bounded; a wait that runs out is reported through ctl->fault) */
     if (p.hot_n) {
-        /* 16-bit passes hold twice the entries in the same bytes */
-        const uint32_t hn = ps.gather_elem_bytes() == 2 ? p.hot_n16 : p.hot_n;
-        const uint32_t bytes = hn * ps.gather_elem_bytes();
+        const uint32_t bytes = p.hot_n * 4;
         if (tid == 0) {
             ag_mbar_init(&s_bar, 1);
             ag_mbar_expect_tx(&s_bar, bytes);
@@ -897,8 +770,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
             ag_mbar_wait(&s_bar, 0, 1u << 24);
         }
         ps.hot32 = reinterpret_cast<const float *>(hot);
-        ps.hot16 = reinterpret_cast<const uint16_t *>(hot);
-        ps.hot_n = hn;
+        ps.hot_n = p.hot_n;
     }
 
     /* each warp walks its tasks with a stride of all warps; the first id
@@ -906,7 +778,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
      * gathered, reduced and written, so it is in flight meanwhile */
     uint32_t t = blockIdx.x * AG_WARPS + warp;
     uint4 task = t < p.ntasks ? p.tasks[t] : make_uint4(0, 0, 0, 0);
-    typename AgPass<MODE, PREC, EXACT, LOW>::Pair pf = ps.prefetch(task.z, task.w, lane);
+    typename AgPass<MODE, EXACT>::Pair pf = ps.prefetch(task.z, task.w, lane);
     AgSteal steal;
     while (t < p.ntasks) {
         uint32_t tn = t + nwarps;
@@ -938,71 +810,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
                 continue;
             }
         }
-        if (MODE == AG_MODE_DD && kind == AG_T_ROWS) {
-            /* data-driven: the sums are those of the plain pull over the
-             * gathered magnitudes; a row is active when the pass is the first
-             * or a gathered value carries the sign of a change */
-            const uint32_t r = r0 + lane;
-            const bool live = r < task.y;
-            uint32_t o0 = ee, o1 = ee, od = 0;
-            float rp = 0.0f;
-            if (live) {
-                o0 = ag_ld_row_u32(p.row_off + r);
-                o1 = ag_ld_row_u32(p.row_off + r + 1);
-                rp = ag_ld_rank(p.rank + r);
-                od = ag_ld_row_u32(p.outdeg + r);
-            }
-            const typename AgPass<MODE, PREC, EXACT, LOW>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
-            ps.stage(vals, eb, ee, lane, pf);
-            __syncwarp();
-            o0 -= eb;
-            o1 -= eb;
-            float s = 0.0f;
-            uint32_t neg = 0;
-            bool is_long = false;
-            if (EXACT) {
-                s = ps.seq_sum(vals, o0, o1, 0.0f, true, neg);
-            } else if (o1 - o0 <= AG_TSEQ) {
-                if (o1 > o0) {
-                    float v = vals[o0];
-                    neg = ps.dd_neg(v);
-                    s = fabsf(v);
-                    for (uint32_t j = o0 + 1; j < o1; ++j) {
-                        v = vals[j];
-                        neg |= ps.dd_neg(v);
-                        s = __fadd_rn(s, fabsf(v));
-                    }
-                }
-            } else {
-                is_long = true;
-            }
-            if (!EXACT) {
-                unsigned m = __ballot_sync(0xffffffffu, is_long);
-                while (m) {
-                    const int src = __ffs(m) - 1;
-                    m &= m - 1;
-                    const uint32_t a = __shfl_sync(0xffffffffu, o0, src);
-                    const uint32_t b = __shfl_sync(0xffffffffu, o1, src);
-                    float tsum = 0.0f;
-                    uint32_t tneg = 0;
-                    for (uint32_t j = a + lane; j < b; j += 32) {
-                        const float v = vals[j];
-                        tneg |= ps.dd_neg(v);
-                        tsum = __fadd_rn(tsum, fabsf(v));
-                    }
-                    tsum = ag_warp_sum_f(tsum);
-                    tneg = __any_sync(0xffffffffu, tneg) ? 1u : 0u;
-                    if ((int)lane == src) {
-                        s = tsum;
-                        neg = tneg;
-                    }
-                }
-            }
-            if (live)
-                ps.finish_dd(r, s, rp, od, ps.dd_all || neg);
-            __syncwarp();
-            pf = pn;
-        } else if (kind == AG_T_ROWS) {
+        if (kind == AG_T_ROWS) {
             /* one row per lane; its bounds, previous rank and out-degree are
              * loaded first so that they arrive while the stage runs */
             const uint32_t r = r0 + lane;
@@ -1017,7 +825,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
                     od = ag_ld_row_u32(p.outdeg + r);
                 }
             }
-            const typename AgPass<MODE, PREC, EXACT, LOW>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
+            const typename AgPass<MODE, EXACT>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
             ps.stage(vals, eb, ee, lane, pf);
             __syncwarp();
             o0 -= eb;
@@ -1026,8 +834,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
             bool is_long = false;
             if (EXACT) {
                 /* stream order, rows of any length: 16-byte shared loads */
-                uint32_t nn = 0;
-                s = ps.seq_sum(vals, o0, o1, 0.0f, true, nn);
+                s = ps.seq_sum(vals, o0, o1, 0.0f, true);
             } else if (o1 - o0 <= AG_TSEQ) {
                 /* stream order: the accumulator restarts with the first value
                  * and adds the rest one by one */
@@ -1067,22 +874,16 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
                 rp = p.rank[r0];
                 od = p.outdeg[r0];
             }
-            const typename AgPass<MODE, PREC, EXACT, LOW>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
+            const typename AgPass<MODE, EXACT>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
             float s;
-            uint32_t neg = 0;
             if (EXACT) {
-                s = ps.ordered_sum(vals, eb, ee, lane, pf, neg);
+                s = ps.ordered_sum(vals, eb, ee, lane, pf);
             } else {
-                s = ps.strided_partial(eb, ee, lane, pf, neg);
+                s = ps.strided_partial(eb, ee, lane, pf);
                 s = ag_warp_sum_f(s);
             }
-            if (MODE == AG_MODE_DD) {
-                const bool act = ps.dd_all || __any_sync(0xffffffffu, neg);
-                if (lane == 0)
-                    ps.finish_dd(r0, s, rp, od, act);
-            } else if (lane == 0) {
+            if (lane == 0)
                 ps.finish(r0, s, rp, od);
-            }
             __syncwarp();
             pf = pn;
         } else if (EXACT) {
@@ -1093,15 +894,11 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
             const uint32_t pbase = task.y & AG_SLOT_MASK, chunk = task.y >> AG_SLOT_BITS;
             const uint32_t o0 = eb - chunk * p.whub;
             float *row_vals = p.hub_vals + (size_t)pbase * p.whub;
-            const typename AgPass<MODE, PREC, EXACT, LOW>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
+            const typename AgPass<MODE, EXACT>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
             if (chunk == 0) {
-                uint32_t neg0 = 0;
-                const float s0 = ps.ordered_sum(vals, eb, ee, lane, pf, neg0);
-                if (lane == 0) {
-                    /* data-driven: the sign bit carries the chunk's tag */
-                    const uint32_t bits = __float_as_uint(s0) | (MODE == AG_MODE_DD && neg0 ? 0x80000000u : 0u);
-                    reinterpret_cast<uint32_t *>(p.hub_part)[pbase] = bits;
-                }
+                const float s0 = ps.ordered_sum(vals, eb, ee, lane, pf);
+                if (lane == 0)
+                    p.hub_part[pbase] = s0;
             } else {
                 const uint32_t pred = __ldcg(p.hub_pred + pbase + chunk);
                 ps.hub_steps(row_vals, o0, eb, ee, lane, pf, pred & 0xffu, ps.hub_staged(pred),
@@ -1128,11 +925,9 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
                         steal.donor = (int)d;
                     }
                 }
-                const typename AgPass<MODE, PREC, EXACT, LOW>::XSum xs = AgPass<MODE, PREC, EXACT, LOW>::hub_compose(
+                const float tot = AgPass<MODE, EXACT>::hub_compose(
                     reinterpret_cast<const uint32_t *>(p.hub_part), p.hub_t, p.hub_pred, row_vals, p.ids, ps.c_in32,
                     vals, p.whub, o0, deg, pbase, nch, lane);
-                const float tot = xs.s;
-                const uint32_t neg = xs.neg;
                 if (lane == 0) {
                     p.hub_cnt[pbase] = 0;
                     float rp = 0.0f;
@@ -1141,10 +936,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
                         rp = p.rank[r0];
                         od = p.outdeg[r0];
                     }
-                    if (MODE == AG_MODE_DD)
-                        ps.finish_dd(r0, tot, rp, od, ps.dd_all || neg);
-                    else
-                        ps.finish(r0, tot, rp, od);
+                    ps.finish(r0, tot, rp, od);
                 }
             }
             __syncwarp();
@@ -1155,14 +947,9 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
             uint32_t deg = 0;
             if (lane == 0)
                 deg = p.row_off[r0 + 1] - p.row_off[r0];
-            const typename AgPass<MODE, PREC, EXACT, LOW>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
-            /* data-driven: each chunk's partial carries the sign of a change
-             * among its in-neighbours; the last chunk ORs them */
-            uint32_t neg = 0;
-            float s = ps.strided_partial(eb, ee, lane, pf, neg);
+            const typename AgPass<MODE, EXACT>::Pair pn = ps.prefetch(task_n.z, task_n.w, lane);
+            float s = ps.strided_partial(eb, ee, lane, pf);
             s = ag_warp_sum_f(s);
-            if (MODE == AG_MODE_DD && __any_sync(0xffffffffu, neg))
-                s = __uint_as_float(__float_as_uint(s) | 0x80000000u);
             if (lane == 0) {
                 const uint32_t nch = (deg + p.whub - 1) / p.whub;
                 p.hub_part[pbase + chunk] = s;
@@ -1171,17 +958,8 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
                 if (prev == nch - 1) {
                     __threadfence();
                     float tot = __ldcg(p.hub_part + pbase);
-                    uint32_t any = 0;
-                    if (MODE == AG_MODE_DD) {
-                        any = ps.dd_neg(tot);
-                        tot = fabsf(tot);
-                    }
-                    for (uint32_t c = 1; c < nch; ++c) {
-                        const float part = __ldcg(p.hub_part + pbase + c);
-                        if (MODE == AG_MODE_DD)
-                            any |= ps.dd_neg(part);
-                        tot = __fadd_rn(tot, MODE == AG_MODE_DD ? fabsf(part) : part);
-                    }
+                    for (uint32_t c = 1; c < nch; ++c)
+                        tot = __fadd_rn(tot, __ldcg(p.hub_part + pbase + c));
                     p.hub_cnt[pbase] = 0;
                     float rp = 0.0f;
                     uint32_t od = 0;
@@ -1189,10 +967,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
                         rp = p.rank[r0];
                         od = p.outdeg[r0];
                     }
-                    if (MODE == AG_MODE_DD)
-                        ps.finish_dd(r0, tot, rp, od, ps.dd_all || any);
-                    else
-                        ps.finish(r0, tot, rp, od);
+                    ps.finish(r0, tot, rp, od);
                 }
             }
             __syncwarp();
@@ -1322,24 +1097,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
             c->hist_err[P] = err;
             c->hist_t[P] = ag_globaltimer();
         }
-        bool conv = (active == 0);
-        if (PREC != 0) {
-            const uint32_t read_low = vc->mode_read;
-            uint32_t next_write = vc->mode_write;
-            if (read_low)
-                c->low_passes = vc->low_passes + 1;
-            /* leave 16-bit storage once the residual is small, once it stops
-             * falling, or once the 16-bit map has reached its fixed point */
-            if (next_write && (err < vc->switch_residual || conv || (P >= 2 && err >= 0.98 * vc->prev_err)))
-                next_write = 0;
-            /* convergence only counts on FP32 contributions */
-            if (read_low)
-                conv = false;
-            c->mode_read = vc->mode_write;
-            c->mode_write = next_write;
-            if (c->mode_read == 0 && vc->switch_pass == 0)
-                c->switch_pass = P + 1;
-        }
+        const bool conv = active == 0;
         c->prev_err = err;
         c->last_err_sum = vc->err_acc;
         c->iter = P + 1;
@@ -1355,7 +1113,7 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
     }
 }
 
-template <int MODE, int PREC, bool EXACT>
+template <int MODE, bool EXACT>
 __global__ void __launch_bounds__(AG_BLK, AG_CTAS_PER_SM) ag_pull_kernel(const AgPullParams p)
 {
     __shared__ double s_redd[AG_WARPS];
@@ -1367,18 +1125,10 @@ __global__ void __launch_bounds__(AG_BLK, AG_CTAS_PER_SM) ag_pull_kernel(const A
      * after the loop has ended return at once */
     if ((MODE != AG_MODE_SPMV || p.honor_stop) && !p.use_cond && *((volatile uint32_t *)&p.ctl->stop))
         return;
-    if constexpr (PREC != 0) {
-        /* the storage this pass reads, set by the pass before */
-        if (*((volatile uint32_t *)&p.ctl->mode_read)) {
-            ag_pull_body<MODE, PREC, EXACT, true>(p, s_redd, s_redu, s_last, s_bar);
-            return;
-        }
-    }
-    ag_pull_body<MODE, PREC, EXACT, false>(p, s_redd, s_redu, s_last, s_bar);
+    ag_pull_body<MODE, EXACT>(p, s_redd, s_redu, s_last, s_bar);
 }
 
 /* init: r = base (or the warm start), first contributions, control reset */
-template <int PREC>
 __global__ void __launch_bounds__(AG_SBLK) ag_pr_init_kernel2(const AgPullParams p, const AgRunConfig run)
 {
     const uint64_t pol_last = ag_policy_evict_last();
@@ -1388,10 +1138,7 @@ __global__ void __launch_bounds__(AG_SBLK) ag_pr_init_kernel2(const AgPullParams
         p.rank[v] = r0;
         const uint32_t od = p.outdeg[v];
         const float c = od ? __fdiv_rn(r0, __uint2float_rn(od)) : 0.0f;
-        if (PREC != 0)
-            ag_st_keep_u16(p.c16_0 + v, ag_f32_to_low<PREC>(c), pol_last);
-        else
-            ag_st_keep_f32(p.c32_0 + p.c_base + v, c, pol_last);
+        ag_st_keep_f32(p.c32_0 + p.c_base + v, c, pol_last);
     }
     for (uint32_t g = blockIdx.x * AG_SBLK + threadIdx.x; g < p.ngraphs; g += gridDim.x * AG_SBLK) {
         p.g_active[g] = 0;
@@ -1410,8 +1157,8 @@ __global__ void __launch_bounds__(AG_SBLK) ag_pr_init_kernel2(const AgPullParams
         c->err_acc = 0.0;
         c->eps = run.eps;
         c->converged = 0;
-        c->mode_read = PREC != 0 ? 1u : 0u;
-        c->mode_write = PREC != 0 ? 1u : 0u;
+        c->mode_read = 0;
+        c->mode_write = 0;
         c->switch_pass = 0;
         c->switch_residual = run.switch_residual;
         c->prev_err = 1e300;
@@ -1513,35 +1260,18 @@ __global__ void ag_f64_fill(uint32_t N, double *r, double v0)
 }
 
 /* ------------------------------------------------------- host glue */
-extern "C" const void *ag_pull_kernel_ptr(int mode, int prec, int exact)
+extern "C" const void *ag_pull_kernel_ptr(int mode, int exact)
 {
     if (mode == AG_MODE_SPMV)
-        return exact ? (const void *)ag_pull_kernel<AG_MODE_SPMV, 0, true>
-                     : (const void *)ag_pull_kernel<AG_MODE_SPMV, 0, false>;
+        return exact ? (const void *)ag_pull_kernel<AG_MODE_SPMV, true>
+                     : (const void *)ag_pull_kernel<AG_MODE_SPMV, false>;
     if (mode == AG_MODE_MULTI)
-        return exact ? (const void *)ag_pull_kernel<AG_MODE_MULTI, 0, true>
-                     : (const void *)ag_pull_kernel<AG_MODE_MULTI, 0, false>;
-    if (mode == AG_MODE_DD)
-        return exact ? (const void *)ag_pull_kernel<AG_MODE_DD, 0, true>
-                     : (const void *)ag_pull_kernel<AG_MODE_DD, 0, false>;
-    switch (prec) {
-    case 1:
-        return exact ? (const void *)ag_pull_kernel<AG_MODE_PR, 1, true> : (const void *)ag_pull_kernel<AG_MODE_PR, 1, false>;
-    case 2:
-        return exact ? (const void *)ag_pull_kernel<AG_MODE_PR, 2, true> : (const void *)ag_pull_kernel<AG_MODE_PR, 2, false>;
-    default:
-        return exact ? (const void *)ag_pull_kernel<AG_MODE_PR, 0, true> : (const void *)ag_pull_kernel<AG_MODE_PR, 0, false>;
-    }
+        return exact ? (const void *)ag_pull_kernel<AG_MODE_MULTI, true>
+                     : (const void *)ag_pull_kernel<AG_MODE_MULTI, false>;
+    return exact ? (const void *)ag_pull_kernel<AG_MODE_PR, true> : (const void *)ag_pull_kernel<AG_MODE_PR, false>;
 }
 
-extern "C" const void *ag_init_kernel_ptr(int prec)
-{
-    switch (prec) {
-    case 1: return (const void *)ag_pr_init_kernel2<1>;
-    case 2: return (const void *)ag_pr_init_kernel2<2>;
-    default: return (const void *)ag_pr_init_kernel2<0>;
-    }
-}
+extern "C" const void *ag_init_kernel_ptr(void) { return (const void *)ag_pr_init_kernel2; }
 
 extern "C" const void *ag_normalize_kernel_ptr(void) { return (const void *)ag_normalize_kernel; }
 

@@ -371,17 +371,20 @@ struct ag_graph_s
     AgControl *ctl;
     float *init_buf;
     uint32_t *flag;
-    /* the solve kernel's bins and its hub rows' state; none (sync NULL) on a
-     * graph that the pull kernel's loop runs */
+    /* the solve kernel's bins or units and its hub rows' state; none (sync
+     * NULL) on a row partition and on a large union */
     AgBinPlan bin;
+    AgUnitPlan unit;
     double *hub_sum;
-    uint32_t *hub_words, *hub_seen;
-    uint8_t *hub_pred8;
+    uint4 *hub_words;
+    uint32_t *hub_seen, *hub_tag;
+    uint16_t *hub_pred16;
+    float4 *hub_kept;
+    uint32_t kept_cap;
     uint32_t *sync;
-    AgExec exe[3][2];
-    int have_exe[3][2];
-    /* data-driven mode: its launch graphs (FAST, EXACT) */
-    AgExec exe_dd[2];
+    /* the pull kernel's loop over a large union (FAST, EXACT) */
+    AgExec exe[2];
+    int have_exe[2];
     /* integer pulls (fixed point and quantised): contribution buffers (the
      * narrow forms use the first N * W/8 bytes), hub partials (capacity in
      * chunks), the quantised forms' binary32 contributions and min/max key
@@ -400,7 +403,6 @@ struct ag_graph_s
     uint8_t *wl;
     AgExec exe_push[AG_NUM_PUSH_FORMS];
     int have_exe_push[AG_NUM_PUSH_FORMS];
-    int have_exe_dd[2];
     cudaEvent_t ev0, ev1;
     int launched;
     int last_prec, last_exact;
@@ -443,16 +445,10 @@ static void free_exec(AgExec *x)
 /* forget every cached launch graph (they carry buffer pointers and tiles) */
 static void drop_execs(ag_graph_s *g)
 {
-    for (int a = 0; a < 3; ++a)
-        for (int b = 0; b < 2; ++b)
-            if (g->have_exe[a][b]) {
-                free_exec(&g->exe[a][b]);
-                g->have_exe[a][b] = 0;
-            }
     for (int b = 0; b < 2; ++b)
-        if (g->have_exe_dd[b]) {
-            free_exec(&g->exe_dd[b]);
-            g->have_exe_dd[b] = 0;
+        if (g->have_exe[b]) {
+            free_exec(&g->exe[b]);
+            g->have_exe[b] = 0;
         }
     for (int b = 0; b < AG_NUM_INT_FORMS; ++b)
         if (g->have_exe_int[b]) {
@@ -519,8 +515,21 @@ extern "C" ag_status_t ag_graph_release(ag_graph_t g)
     dev_free(g->bin.tmp);
     dev_free(g->hub_sum);
     dev_free(g->hub_words);
+    dev_free(g->unit.info);
+    dev_free(g->unit.ubase);
+    dev_free(g->unit.heavy);
+    dev_free(g->unit.bstart);
+    dev_free(g->unit.outdeg);
+    dev_free(g->unit.posof);
+    dev_free(g->unit.hubs);
+    dev_free(g->unit.hrow);
+    dev_free(g->unit.ids);
+    dev_free(g->unit.cnt);
+    dev_free(g->unit.tmp);
+    dev_free(g->hub_tag);
     dev_free(g->hub_seen);
-    dev_free(g->hub_pred8);
+    dev_free(g->hub_pred16);
+    dev_free(g->hub_kept);
     dev_free(g->sync);
     dev_free(g->ctl);
     dev_free(g->init_buf);
@@ -627,15 +636,16 @@ static ag_status_t plan_device(ag_graph_s *g, uint32_t cap, uint32_t whub)
     return AG_OK;
 }
 
-/* Graphs of more in-edges run on the pull kernel's loop: there the solve
- * kernel's bins wait longer for their gathers than the pull kernel's warps,
- * which overlap theirs item by item.  us per pass, pull kernel / solve kernel
- * (EXACT; R-MAT, 16 edges per vertex): 54 / 21 at 1 M in-edges, 127 / 83 at
- * 16 M, 130 / 91 at 18 M, but 336 / 348 at 65 M; FAST order 20 / 13, 65.8 /
- * 66.4, 81 / 79, 218 / 295. */
-#ifndef AG_BIN_MAX_EDGES
-#define AG_BIN_MAX_EDGES 20000000u
-#endif
+/* Whole graphs from here on run as units, smaller ones as bins.  us per pass,
+ * units / bins, FAST and EXACT: 10.8 M in-edges (uniform) 62 / 57 and 63 / 57;
+ * 16 M (R-MAT) 63 / 66 and 97 / 72; 17 M (R-MAT, 900 K vertices) 67 / 75 and
+ * 87 / 97; 21 M (uniform) 100 / 107 and 100 / 108; 33 M (R-MAT) 98 / 127 and
+ * 125 / 148; 65 M (R-MAT) 183 / 265 and 232 / 300. */
+#define AG_UNIT_MIN_EDGES 17000000u
+/* Unions above this stay on the pull kernel's loop, one launch per pass: their
+ * bins gather from L2 alone.  us per pass, pull kernel / bins, FAST and EXACT:
+ * 30 M in-edges 205 / 185 and 228 / 175, 124 M 806 / 900 and 854 / 887. */
+#define AG_UNION_MAX_EDGES 64000000u
 /* Row weight per bin: one bin for every group of the persistent grid on a
  * small graph, several of at most AG_BIN_QUANTUM on a larger one (the same
  * number for each group).  A larger bin has fewer waits, a smaller one leaves
@@ -669,9 +679,12 @@ static ag_status_t plan_bins(ag_graph_s *g, uint64_t total)
     b->ubase = (uint32_t *)dev_alloc(g, words / 32 * 4 + 16, &st);
     b->ids = (uint32_t *)dev_alloc(g, (size_t)b->nslots * 4, &st);
     g->hub_sum = (double *)dev_alloc(g, (size_t)b->nhub * 8, &st);
-    g->hub_words = (uint32_t *)dev_alloc(g, (size_t)b->nhub * AG_BIN_ROUNDS * 4, &st);
+    g->hub_words = (uint4 *)dev_alloc(g, (size_t)b->nhub * AG_BIN_ROUNDS * 16, &st);
     g->hub_seen = (uint32_t *)dev_alloc(g, (size_t)b->nhub * 4, &st);
-    g->hub_pred8 = (uint8_t *)dev_alloc(g, (size_t)b->nhub * AG_BIN_ROUNDS, &st);
+    /* (a chunk reads up to two entries past its own) */
+    g->hub_pred16 = (uint16_t *)dev_alloc(g, (size_t)b->nhub * AG_BIN_ROUNDS * 2 + 16, &st);
+    g->kept_cap = 2 * b->nhub;
+    g->hub_kept = (float4 *)dev_alloc(g, (size_t)g->kept_cap * AG_KEPT_QUADS * 16, &st);
     g->sync = (uint32_t *)dev_alloc(g, AG_SYNC_WORDS * 4, &st);
     if (st != AG_OK)
         return st;
@@ -685,6 +698,74 @@ static ag_status_t plan_bins(ag_graph_s *g, uint64_t total)
         return ag_set_error(AG_ERR_CUDA, "bin planning failed: %s", cudaGetErrorString(e));
     }
     return AG_OK;
+}
+
+/* whether the solve kernel runs this graph as units (else as bins) */
+static bool want_units(const ag_graph_s *g)
+{
+    /* quads are counted in 32 bits: padding is below one quad a row and 32 x
+     * AG_UNIT_LONG / 4 a window */
+    const uint64_t quads = g->E / 4u + (uint64_t)g->N + ((uint64_t)g->N / AG_UNIT_WIN + 1) * (8 * AG_UNIT_LONG);
+    return !g->ngraphs && g->E >= AG_UNIT_MIN_EDGES && quads < (1ull << 32);
+}
+
+static ag_status_t plan_unit_rows(ag_graph_s *g, uint32_t *totals)
+{
+    AgUnitPlan *u = &g->unit;
+    ag_status_t st = AG_OK;
+    const size_t nu = ((size_t)g->N + 31) / 32;
+    u->info = (uint32_t *)dev_alloc(g, (size_t)g->N * 4, &st);
+    u->ubase = (uint32_t *)dev_alloc(g, (nu + 1) * 4, &st);
+    /* Quads per row that a warp adds in a pass.  The longest row of a unit is a
+     * chain of gathers, about 0.75 us per eight in-edges: it should end well
+     * inside the pass.  us per pass (FAST / EXACT) with 512, 768 or 1024, 2047:
+     * 33 M in-edges 98 / 135, 145 / 166, 143 / 163; 65 M 190 / 248, 182 / 231,
+     * 245 / 263; 263 M 798 / 993, 796 / 988, 761 / 881.  Units of a quarter of
+     * that share or more run first.  Batches of weight 8, 16, 32, 64: 106 / 140,
+     * 101 / 128, 108 / 136, 133 / 153 at 33 M; 198 / 246, 189 / 235, 199 / 243,
+     * 211 / 251 at 65 M. */
+    const uint64_t share = g->E / 128u / ((uint64_t)std::max(1, g_ctx.num_sms) * (AG_SOLVE_BLK / 32));
+    u->longest = (uint32_t)std::min<uint64_t>(AG_UNIT_LONG, std::max<uint64_t>(AG_BIN_HEAD, 7 * share));
+    u->heavy_quads = (uint32_t)std::min<uint64_t>(64, std::max<uint64_t>(16, share / 4));
+    u->batch = 16;
+    u->heavy = (uint32_t *)dev_alloc(g, nu * 4, &st);
+    u->outdeg = (uint32_t *)dev_alloc(g, (size_t)g->N * 4, &st);
+    u->posof = (uint32_t *)dev_alloc(g, (size_t)g->N * 4, &st);
+    u->cnt = (uint32_t *)dev_alloc(g, 16, &st);
+    g->sync = (uint32_t *)dev_alloc(g, AG_SYNC_WORDS * 4, &st);
+    if (st != AG_OK)
+        return st;
+    cudaError_t e = ag_units_rows(g->row_off, g->outdeg, g->N, u, totals, g_ctx.stream);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(g->sync, 0, AG_SYNC_WORDS * 4, g_ctx.stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return ag_set_error(AG_ERR_CUDA, "unit planning failed: %s", cudaGetErrorString(e));
+    }
+    return AG_OK;
+}
+
+static ag_status_t plan_unit_ids(ag_graph_s *g, const uint32_t *totals)
+{
+    AgUnitPlan *u = &g->unit;
+    ag_status_t st = AG_OK;
+    u->nhub = totals[0];
+    u->nhrow = totals[1];
+    u->nheavy = totals[2];
+    u->quads = totals[3];
+    u->nbatch = ag_units_batches(u, u->quads);
+    u->bstart = (uint32_t *)dev_alloc(g, ((size_t)u->nbatch + 1) * 4, &st);
+    u->hubs = (uint4 *)dev_alloc(g, (size_t)u->nhub * sizeof(uint4), &st);
+    u->hrow = (uint32_t *)dev_alloc(g, (size_t)u->nhrow * 4, &st);
+    u->ids = (uint4 *)dev_alloc(g, ((size_t)u->nhub * (AG_BIN_HUB / 4) + u->quads) * 16, &st);
+    g->hub_sum = (double *)dev_alloc(g, (size_t)u->nhub * 8, &st);
+    g->hub_words = (uint4 *)dev_alloc(g, (size_t)u->nhub * AG_BIN_ROUNDS * 16, &st);
+    /* (a chunk reads up to two entries past its own) */
+    g->hub_pred16 = (uint16_t *)dev_alloc(g, (size_t)u->nhub * AG_BIN_ROUNDS * 2 + 16, &st);
+    g->kept_cap = 2 * u->nhub;
+    g->hub_kept = (float4 *)dev_alloc(g, (size_t)g->kept_cap * AG_KEPT_QUADS * 16, &st);
+    g->hub_tag = (uint32_t *)dev_alloc(g, (size_t)u->nhub * 8, &st);
+    return st;
 }
 
 static ag_status_t upload_impl(const struct GraphCSR *graph, uint32_t flags, const uint32_t *gstart_host,
@@ -966,14 +1047,18 @@ static ag_status_t upload_impl(const struct GraphCSR *graph, uint32_t flags, con
             UPFAIL(st);
         UP(cudaMemcpyAsync(g->gstart, gstart_host, (size_t)(ngraphs + 1) * 4, cudaMemcpyHostToDevice, s));
     }
-    /* a row partition runs pass by pass on the pull kernel, without bins */
-    const bool bins = gather_n == 0 && E <= AG_BIN_MAX_EDGES;
+    /* a row partition and a large union run pass by pass on the pull kernel */
+    const bool whole = gather_n == 0 && !(ngraphs && E > AG_UNION_MAX_EDGES), units = whole && want_units(g);
     uint64_t bin_total = 0;
-    if (bins)
+    uint32_t unit_totals[4] = {0, 0, 0, 0};
+    if (units)
+        st = plan_unit_rows(g, unit_totals);
+    else if (whole)
         UP(ag_bins_count(g->row_off, N, &g->bin, &bin_total, s));
-    st = plan_device(g, g->tiles.task_edges, g->tiles.hub_chunk);
-    if (st == AG_OK && bins)
-        st = plan_bins(g, bin_total);
+    if (st == AG_OK)
+        st = plan_device(g, g->tiles.task_edges, g->tiles.hub_chunk);
+    if (st == AG_OK && whole)
+        st = units ? plan_unit_ids(g, unit_totals) : plan_bins(g, bin_total);
     if (st != AG_OK)
         UPFAIL(st);
 
@@ -1009,7 +1094,11 @@ static ag_status_t upload_impl(const struct GraphCSR *graph, uint32_t flags, con
         off_old = ids_old = outdeg_old = nullptr;
         w_old = nullptr;
     }
-    if (bins) {
+    if (units) {
+        UP(ag_units_ids(g->row_off, g->ids, N, &g->unit, s));
+        dev_free(g->unit.tmp);
+        g->unit.tmp = nullptr;
+    } else if (whole) {
         UP(ag_bins_ids(g->row_off, g->ids, &g->bin, s));
         dev_free(g->bin.pre);
         dev_free(g->bin.tmp);
@@ -1045,8 +1134,8 @@ extern "C" ag_status_t ag_graph_get_info(ag_graph_t g, ag_graph_info *info)
     info->max_in_degree = g->max_in_degree;
     info->device_bytes = g->device_bytes;
     int nb = 0;
-    if (pull_kernel_prepare(ag_pull_kernel_ptr(AG_MODE_PR, 0, 0), pull_smem(g)) == AG_OK &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ag_pull_kernel_ptr(AG_MODE_PR, 0, 0), AG_BLK,
+    if (pull_kernel_prepare(ag_pull_kernel_ptr(AG_MODE_PR, 0), pull_smem(g)) == AG_OK &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ag_pull_kernel_ptr(AG_MODE_PR, 0), AG_BLK,
                                                       pull_smem(g)) == cudaSuccess)
         info->grid = (uint32_t)std::min<uint64_t>((uint64_t)nb * g_ctx.num_sms,
                                                   std::max<uint64_t>(1, ((uint64_t)g->ntasks_fast + AG_WARPS - 1) / AG_WARPS));
@@ -1178,19 +1267,14 @@ static AgPullParams base_params(ag_graph_s *g, int exact)
     return p;
 }
 
-static int pull_mode(const ag_graph_s *g, int dd)
-{
-    return dd ? AG_MODE_DD : (g->ngraphs ? AG_MODE_MULTI : AG_MODE_PR);
-}
-
-/* the solve's kernels: pull, init and (quantised forms) quantise */
-static const void *solve_pull_kernel(const ag_graph_s *g, int prec, int exact, int dd)
+/* the loop's kernels: an integer form's, or the pull kernel's over a union */
+static const void *loop_pull_kernel(int prec, int exact)
 {
     return is_int_prec(prec) ? ag_int_kernel_ptr(int_bytes(prec), int_quant(prec), 0)
-                             : ag_pull_kernel_ptr(pull_mode(g, dd), prec, exact);
+                             : ag_pull_kernel_ptr(AG_MODE_MULTI, exact);
 }
 
-static size_t solve_smem(const ag_graph_s *g, int prec)
+static size_t loop_smem(const ag_graph_s *g, int prec)
 {
     return is_int_prec(prec) ? ag_fixed_smem_bytes(int_bytes(prec)) : pull_smem(g);
 }
@@ -1219,21 +1303,47 @@ static ag_status_t solve_launch(ag_graph_s *g, int prec, int exact, int dd, cons
     q.nhb = (q.nhub + q.per_bin - 1) / q.per_bin;
     q.hub_sum = g->hub_sum;
     q.hub_words = g->hub_words;
-    q.hub_pred = g->hub_pred8;
+    q.hub_pred = g->hub_pred16;
+    q.kept = g->hub_kept;
+    q.kept_cap = g->kept_cap;
     q.hub_seen = g->hub_seen;
     q.sync = g->sync;
     q.spins = AG_GRID_SPINS;
-    const size_t bufs = (size_t)AG_SUBS * q.buf * 4;
+    size_t bufs = (size_t)AG_SUBS * q.buf * 4;
+    uint64_t work = (uint64_t)q.nhb + q.nbins;
+    if (g->unit.nunits) {
+        const AgUnitPlan &u = g->unit;
+        q.nunits = u.nunits;
+        q.nhrow = u.nhrow;
+        q.nheavy = u.nheavy;
+        q.heavy = u.heavy;
+        q.heavy_quads = u.heavy_quads;
+        q.nbatch = u.nbatch;
+        q.bstart = u.bstart;
+        q.nhub = u.nhub;
+        q.info = u.info;
+        q.uoutdeg = u.outdeg;
+        q.posof = u.posof;
+        q.hrow = u.hrow;
+        q.ubaseq = u.ubase;
+        q.hubs = u.hubs;
+        q.ids = (const uint32_t *)u.ids;
+        q.uids = u.ids + (size_t)u.nhub * (AG_BIN_HUB / 4);
+        q.hub_tag = g->hub_tag;
+        bufs = 0;
+        work = q.nunits;
+    }
     const uint32_t fit = (uint32_t)((AG_SMEM_MAX - AG_SMEM_STATIC - bufs) / 4) & ~63u;
     q.p.hot_n = std::min(q.p.hot_n, fit);
     q.p.hot_n16 = std::min<uint32_t>(2 * q.p.hot_n, g->N & ~63u);
     const size_t smem = (size_t)q.p.hot_n * 4 + bufs;
-    const void *k = ag_solve_kernel_ptr(dd ? AG_MODE_DD : g->ngraphs ? AG_MODE_MULTI : AG_MODE_PR, prec, exact);
+    const void *k = ag_solve_kernel_ptr(dd ? AG_MODE_DD : g->ngraphs ? AG_MODE_MULTI : AG_MODE_PR, prec, exact,
+                                        q.nunits != 0);
     ag_status_t st = pull_kernel_prepare(k, smem);
     if (st != AG_OK)
         return st;
     const unsigned grid = (unsigned)std::max<uint64_t>(
-        1, std::min<uint64_t>((uint64_t)g_ctx.num_sms, (uint64_t)q.nhb + q.nbins));
+        1, std::min<uint64_t>((uint64_t)g_ctx.num_sms, work));
     AgRunConfig r = run;
     void *args[2] = {&q, &r};
     const char *mode = getenv("AG_LAUNCH_MODE");
@@ -1272,23 +1382,26 @@ static dim3 quant_grid(const ag_graph_s *g)
 }
 
 /* prec: AG_PREC_* (the integer forms take both orders through one graph) */
-static AgExec *exec_slot(ag_graph_s *g, int prec, int exact, int dd)
+static AgExec *exec_slot(ag_graph_s *g, int prec, int exact, int **have)
 {
-    return is_int_prec(prec) ? &g->exe_int[prec - AG_PREC_FIXED64] : dd ? &g->exe_dd[exact] : &g->exe[prec][exact];
+    const int i = prec - AG_PREC_FIXED64;
+    *have = is_int_prec(prec) ? &g->have_exe_int[i] : &g->have_exe[exact];
+    return is_int_prec(prec) ? &g->exe_int[i] : &g->exe[exact];
 }
 
-static ag_status_t build_exec(ag_graph_s *g, int prec, int exact, int dd = 0)
+static ag_status_t build_exec(ag_graph_s *g, int prec, int exact)
 {
     const int ip = is_int_prec(prec), quant = ip && int_quant(prec);
-    AgExec *x = exec_slot(g, prec, exact, dd);
+    int *have;
+    AgExec *x = exec_slot(g, prec, exact, &have);
     memset(x, 0, sizeof(*x));
     AG_CUDA(cudaGraphCreate(&x->graph, 0));
     AG_CUDA(cudaGraphConditionalHandleCreate(&x->cond, x->graph, 1, cudaGraphCondAssignDefault));
     x->params = base_params(g, exact);
     x->params.cond = x->cond;
     x->params.use_cond = 1;
-    const void *kpull = solve_pull_kernel(g, prec, exact, dd);
-    const size_t smem = solve_smem(g, prec);
+    const void *kpull = loop_pull_kernel(prec, exact);
+    const size_t smem = loop_smem(g, prec);
     x->grid = pull_grid(kpull, x->params.ntasks, smem);
 
     /* quantised forms: both min/max slots cleared before the init kernel
@@ -1313,7 +1426,7 @@ static ag_status_t build_exec(ag_graph_s *g, int prec, int exact, int dd = 0)
     memset(&run, 0, sizeof(run));
     void *init_args[2] = {&x->params, &run};
     cudaKernelNodeParams kp = {};
-    kp.func = (void *)(ip ? ag_int_init_kernel_ptr(int_bytes(prec), quant) : ag_init_kernel_ptr(prec));
+    kp.func = (void *)(ip ? ag_int_init_kernel_ptr(int_bytes(prec), quant) : ag_init_kernel_ptr());
     kp.gridDim = elem_grid(g);
     kp.blockDim = dim3(AG_SBLK);
     kp.kernelParams = init_args;
@@ -1358,20 +1471,8 @@ static ag_status_t build_exec(ag_graph_s *g, int prec, int exact, int dd = 0)
     AG_CUDA(cudaGraphAddKernelNode(&nnode, x->graph, &wnode, 1, &kn));
 
     AG_CUDA(cudaGraphInstantiate(&x->exec, x->graph, 0));
-    if (ip)
-        g->have_exe_int[prec - AG_PREC_FIXED64] = 1;
-    else if (dd)
-        g->have_exe_dd[exact] = 1;
-    else
-        g->have_exe[prec][exact] = 1;
+    *have = 1;
     return AG_OK;
-}
-
-static int have_exec(const ag_graph_s *g, int prec, int exact, int dd)
-{
-    return is_int_prec(prec) ? g->have_exe_int[prec - AG_PREC_FIXED64]
-           : dd              ? g->have_exe_dd[exact]
-                             : g->have_exe[prec][exact];
 }
 
 /* integer pull buffers, made on first use; the hub partials follow the
@@ -1528,7 +1629,7 @@ static ag_status_t build_exec_push(ag_graph_s *g, int kind)
         cudaGraphNode_t nseed, nspmv;
         AG_CUDA(cudaGraphAddKernelNode(&nseed, x->graph, nullptr, 0, &ks));
         void *sargs[1] = {&seed_spmv};
-        const void *ksp = ag_pull_kernel_ptr(AG_MODE_SPMV, 0, 1);
+        const void *ksp = ag_pull_kernel_ptr(AG_MODE_SPMV, 1);
         const size_t ssm = push_spmv_smem(seed_spmv);
         if (seed_spmv.ntasks) {
             cudaKernelNodeParams kv = {};
@@ -1580,7 +1681,7 @@ static ag_status_t build_exec_push(ag_graph_s *g, int kind)
     if (kind == AG_PUSH_QUANT)
         AG_CUDA(add(ag_push_kernel_ptr(kind, 3), eg, blk, 0, pargs));
     if (kind == AG_PUSH_PULLPUSH && loop_spmv.ntasks) {
-        const void *ksp = ag_pull_kernel_ptr(AG_MODE_SPMV, 0, 0);
+        const void *ksp = ag_pull_kernel_ptr(AG_MODE_SPMV, 0);
         const size_t lsm = push_spmv_smem(loop_spmv);
         AG_CUDA(add(ksp, dim3(pull_grid(ksp, loop_spmv.ntasks, lsm)), dim3(AG_BLK), lsm, largs));
     }
@@ -1624,7 +1725,7 @@ static ag_status_t push_stream_launch(ag_graph_s *g, int kind, const AgRunConfig
     AgPullParams seed_spmv = push_spmv_params(g, 1), loop_spmv = push_spmv_params(g, 0);
     seed_spmv.honor_stop = 0;
     void *sa[1] = {&seed_spmv}, *la[1] = {&loop_spmv};
-    const void *kse = ag_pull_kernel_ptr(AG_MODE_SPMV, 0, 1), *ksl = ag_pull_kernel_ptr(AG_MODE_SPMV, 0, 0);
+    const void *kse = ag_pull_kernel_ptr(AG_MODE_SPMV, 1), *ksl = ag_pull_kernel_ptr(AG_MODE_SPMV, 0);
     PushScatterShape sh;
     ag_status_t sst = push_scatter_shape(kind, &sh);
     if (sst != AG_OK)
@@ -1784,12 +1885,6 @@ extern "C" ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations,
         /* rebuild cached graphs: their parameters carry the warm-start pointer */
         drop_execs(g);
     }
-    const bool bins = !ip && g->sync;
-    if (!bins && !have_exec(g, prec, exact, dd)) {
-        st = build_exec(g, prec, exact, dd);
-        if (st != AG_OK)
-            return st;
-    }
     cudaStream_t s = g_ctx.stream;
     if (o.init_ranks && g->N)
         AG_CUDA(cudaMemcpyAsync(g->init_buf, o.init_ranks, (size_t)g->N * 4,
@@ -1800,7 +1895,7 @@ extern "C" ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations,
     run.use_init = o.init_ranks ? 1u : 0u;
     run.eps = epsilon;
     run.switch_residual = o.switch_residual > 0 ? o.switch_residual : 1e-4;
-    if (bins) {
+    if (!ip && g->sync) {
         AG_CUDA(cudaEventRecord(g->ev0, s));
         st = solve_launch(g, prec, exact, dd, run);
         if (st != AG_OK)
@@ -1811,7 +1906,13 @@ extern "C" ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations,
         g->last_exact = exact;
         return AG_OK;
     }
-    AgExec *x = exec_slot(g, prec, exact, dd);
+    int *have;
+    AgExec *x = exec_slot(g, prec, exact, &have);
+    if (!*have) {
+        st = build_exec(g, prec, exact);
+        if (st != AG_OK)
+            return st;
+    }
     void *init_args[2] = {&x->params, &run};
     cudaKernelNodeParams kp;
     AG_CUDA(cudaGraphKernelNodeGetParams(x->init_node, &kp));
@@ -1833,8 +1934,8 @@ extern "C" ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations,
         }
         AG_CUDA(cudaLaunchKernel(ki.func, ki.gridDim, ki.blockDim, ia, 0, s));
         void *pa[1] = {&sp};
-        const void *kpull = solve_pull_kernel(g, prec, exact, dd);
-        const size_t smem = solve_smem(g, prec);
+        const void *kpull = loop_pull_kernel(prec, exact);
+        const size_t smem = loop_smem(g, prec);
         for (uint32_t i = 0; i < run.max_iter; ++i) {
             if (quant)
                 AG_CUDA(cudaLaunchKernel(ag_quant_kernel_ptr(int_bytes(prec)), quant_grid(g), dim3(AG_SBLK), pa, 0, s));
@@ -1947,7 +2048,7 @@ extern "C" ag_status_t ag_spmv_pull_device(ag_graph_t g, const float *x, float *
     if (((uintptr_t)p.x & 15u) != 0)
         p.hot_n = 0;
     p.wmode = (mode & AG_SPMV_UNIT) ? AG_SPMV_W_UNIT : (g->w ? AG_SPMV_W_GRAPH : AG_SPMV_W_CONST);
-    const void *k = ag_pull_kernel_ptr(AG_MODE_SPMV, 0, exact);
+    const void *k = ag_pull_kernel_ptr(AG_MODE_SPMV, exact);
     const size_t smem = (size_t)AG_STAGE_BYTES + (size_t)p.hot_n * 4;
     const unsigned grid = pull_grid(k, p.ntasks, smem);
     void *args[1] = {&p};
@@ -2429,7 +2530,7 @@ extern "C" ag_status_t ag_partition_init(ag_graph_t g, float *c_full)
     void *args[2] = {&p, &run};
     const unsigned grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>(((uint64_t)g->N + AG_SBLK - 1) / AG_SBLK, (uint64_t)g_ctx.num_sms * 8));
-    AG_CUDA(cudaLaunchKernel(ag_init_kernel_ptr(0), dim3(grid), dim3(AG_SBLK), args, 0, g_ctx.stream));
+    AG_CUDA(cudaLaunchKernel(ag_init_kernel_ptr(), dim3(grid), dim3(AG_SBLK), args, 0, g_ctx.stream));
     return AG_OK;
 }
 
@@ -2470,7 +2571,7 @@ extern "C" ag_status_t ag_partition_pass(ag_graph_t g, const float *c_in_full, f
         p.c32_0 = const_cast<float *>(c_in_full);
         p.c32_1 = c_out_full;
         p.use_cond = 0;
-        const void *k = ag_pull_kernel_ptr(AG_MODE_PR, 0, 0);
+        const void *k = ag_pull_kernel_ptr(AG_MODE_PR, 0);
         const unsigned grid = pull_grid(k, p.ntasks, pull_smem(g));
         void *args[1] = {&p};
         AG_CUDA(cudaLaunchKernel(k, dim3(grid), dim3(AG_BLK), args, pull_smem(g), s));
@@ -2526,7 +2627,7 @@ extern "C" ag_status_t ag_partition_step(ag_graph_t g, const float *c_in_full, f
         p.c32_0 = const_cast<float *>(c_in_full);
         p.c32_1 = c_out_full;
         p.use_cond = 0;
-        const void *k = ag_pull_kernel_ptr(AG_MODE_PR, 0, exact);
+        const void *k = ag_pull_kernel_ptr(AG_MODE_PR, exact);
         const unsigned grid = pull_grid(k, p.ntasks, pull_smem(g));
         void *args[1] = {&p};
         AG_CUDA(cudaLaunchKernel(k, dim3(grid), dim3(AG_BLK), args, pull_smem(g), s));

@@ -13,9 +13,10 @@
  * pass and the normalisation, with a grid barrier between them: the last CTA
  * to arrive closes the pass (record, stop test) and releases the others.
  *
- * A CTA's warps form AG_SUBS groups, each with its own shared-memory buffer.
- * A group takes one bin at a time (ag_bins.h; hub chunks first, then row bins
- * in row order, handed out by an atomic counter):
+ * Bins (ag_bins.h; graphs up to AG_UNIT_MIN_EDGES, and unions).  A CTA's warps
+ * form AG_SUBS groups, each with its own shared-memory buffer.  A group takes
+ * one bin at a time (hub chunks first, then row bins in row order, handed out
+ * by an atomic counter):
  *   stage   every thread loads four slot ids at a time and gathers their
  *           contributions into the buffer, from the CTA's copy of the most-read
  *           ones (hot table) or from L1 / L2;
@@ -24,23 +25,33 @@
  *   update  the group's rows in row order, coalesced.
  * While one group waits for its gathers the other sums.
  *
+ * Units (ag_units.h; larger graphs).  A warp takes 32 rows of about the same
+ * length, one per lane; each lane gathers eight values of its row at a time
+ * into registers and adds them in stream order, while the next ids travel.
+ * No warp waits for another inside a pass.  Items are handed out by one atomic
+ * counter, those with the longest chains first.
+ *
  * EXACT order: every row is summed in stream order (a hub row as described at
- * exact_round).  FAST order: rows of up to 32 in-edges in stream order; longer
+ * ag_sv_moves).  FAST order: rows of up to 32 in-edges in stream order; longer
  * ones as binary32 trees of eight values added in binary64.
  * Data-driven passes (the reference's worklist pull, pageRank.c:2810-2969): a
  * vertex that changes writes its next contribution with the sign bit set; a
  * row sums magnitudes and is on the worklist when the pass is the first or a
  * sign was set.
- * No result depends on which group ran a bin.
+ * No result depends on which warp ran what.
  *
  * What bounds a pass: on a small graph the chain of waits (barrier, bin, ids,
  * gathers, the longest row's adds, update), about 7 us at 1024 vertices, where
  * the pull kernel's loop, one launch per pass, took 14.5 (EXACT); from a
  * million in-edges on the gathers' L1 misses (about one per SM clock), and in
- * EXACT order the longest rows' chains: 53.8 -> 21.3 us a pass at 65 K
- * vertices and 1 M in-edges, 126.9 -> 82.9 at 1 M vertices and 16 M in-edges
- * (R-MAT).  The pull kernel's EXACT order adds a long row on one lane while
- * the other 31 wait; here they add other rows.
+ * EXACT order what the hub rows add.  us per pass, FAST and EXACT, pull
+ * kernel's loop -> here (R-MAT, 16 edges per vertex): 65 K vertices 19.9 ->
+ * 12.9 and 53.8 -> 17.3; 1 M 65.9 -> 66.3 and 127 -> 71.6; 2 M 115 -> 98 and
+ * 190 -> 125; 4 M 221 -> 183 and 328 -> 232; 8 M 473 -> 380 and 718 -> 470;
+ * 16 M 922 -> 778 and 1332 -> 897 (4E + 24N bytes: 17 -> 25 % of the measured
+ * copy rate).  The pull kernel's EXACT order
+ * adds a long row on one lane while the other 31 wait; here they add other
+ * rows, and neighbouring rows' warps share L1 lines.
  */
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -134,7 +145,7 @@ struct AgSvShared
     uint32_t redu[AG_SOLVE_BLK / 32];
     uint64_t mbar;
     uint32_t last, gen, next[AG_SUBS];
-    uint8_t pred[AG_SUBS][16 * AG_BIN_ROUNDS];
+    uint16_t pred[AG_SUBS][16 * AG_BIN_ROUNDS + 1];
 };
 
 /* ------------------------------------------------------------ exact sums */
@@ -271,36 +282,32 @@ template <int MODE> __device__ __forceinline__ float ag_sv_fast(const float *val
     return __double2float_rn(t);
 }
 
-/* one round of a hub row on the whole warp: the stream-order sum of
- * vals[0, n), n <= 256, continuing s (the same in every lane, as is the
- * result).  The lane where s leaves its binade adds its own eight values in
- * binary32, and the lanes after it start again in the new binade. */
-template <int MODE>
-__device__ __noinline__ float ag_sv_round(const float *vals, uint32_t n, float s, uint32_t lane)
+/* one round of a hub row on the whole warp: the stream-order sum of 256
+ * values, eight consecutive ones per lane (0 past the row's end), continuing s
+ * (the same in every lane, as is the result).  The lane where s leaves its
+ * binade adds its own eight values in binary32, and the lanes after it start
+ * again in the new binade. */
+__device__ __noinline__ float ag_sv_round(float v0, float v1, float v2, float v3, float v4, float v5, float v6, float v7,
+                                          float s, uint32_t lane, uint32_t done)
 {
-    float v[8];
-    ag_sv_eight<MODE>(vals, n, lane, v);
-    for (uint32_t done = 0; done < 32u;) { /* lanes below `done` are in s */
+    const float v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
+    while (done < 32u) { /* lanes below `done` are in s */
         const uint32_t sb = __float_as_uint(s), ex = sb >> 23;
-        if (ex < 24u || ex > 254u) {
-            /* zero, tiny, negative or not finite: one value after another */
-            if (lane == 0)
-                for (uint32_t j = 8u * done; j < n; ++j)
-                    s = __fadd_rn(s, MODE == AG_MODE_DD ? fabsf(vals[j]) : vals[j]);
-            return __shfl_sync(0xffffffffu, s, 0);
-        }
-        const uint32_t m = (sb & 0x7fffffu) | 0x800000u;
-        uint32_t d0 = 0, d1 = 0;
-        if (lane >= done)
-            ag_sv_moves(v, ex, d0, d1);
-        ag_sv_scan(lane, d0, d1);
-        const uint32_t to = m + ((m & 1u) ? d1 : d0);
-        const uint32_t ok = __ballot_sync(0xffffffffu, to < (1u << 24));
-        if (ok == 0xffffffffu)
-            return ag_sv_make(ex, __shfl_sync(0xffffffffu, to, 31));
-        const uint32_t out = __ffs(~ok) - 1;
-        const uint32_t before = __shfl_sync(0xffffffffu, to, (out - 1u) & 31u);
-        s = ag_sv_make(ex, out ? before : m);
+        uint32_t out = done;
+        if (ex >= 24u && ex <= 254u) {
+            const uint32_t m = (sb & 0x7fffffu) | 0x800000u;
+            uint32_t d0 = 0, d1 = 0;
+            if (lane >= done)
+                ag_sv_moves(v, ex, d0, d1);
+            ag_sv_scan(lane, d0, d1);
+            const uint32_t to = m + ((m & 1u) ? d1 : d0);
+            const uint32_t ok = __ballot_sync(0xffffffffu, to < (1u << 24));
+            if (ok == 0xffffffffu)
+                return ag_sv_make(ex, __shfl_sync(0xffffffffu, to, 31));
+            out = __ffs(~ok) - 1;
+            const uint32_t before = __shfl_sync(0xffffffffu, to, (out - 1u) & 31u);
+            s = ag_sv_make(ex, out ? before : m);
+        } /* else zero, tiny, negative or not finite: one lane after another */
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             s = __fadd_rn(s, v[i]);
@@ -317,8 +324,21 @@ __device__ __forceinline__ uint32_t ag_sv_pack(uint32_t d0, uint32_t d1)
     return d0 >= (1u << 24) || d1 >= (1u << 24) ? AG_XNOT : d0 | ((d1 + 1u - d0) << 26);
 }
 
+/* Each round is mapped at two neighbouring exponents, this one and the next:
+ * those nearest to where its sum began in the pass before (`pred`, the top
+ * half of its bits), so that a sum that moved by less than 41 % still finds
+ * its map, or the two that it passes through when the round after it began
+ * (`next`) in a higher binade */
+__device__ __forceinline__ uint32_t ag_sv_low_exp(uint32_t pred, uint32_t next)
+{
+    const uint32_t e = pred >> 7;
+    return (pred & 0x7fu) >= 53u || (next >> 7) > e || e == 0u ? e : e - 1u;
+}
+
+#define AG_SV_NOT_KEPT 0xffffffffu
+
 /* ------------------------------------------------------------------ solve */
-template <int MODE, int PREC, bool EXACT> struct AgSolve
+template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
 {
     const AgSolveParams &q;
     const AgPullParams &p;
@@ -374,6 +394,7 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
                 const uint32_t g = (((gen >> 3) + 1u) << 3) | f;
                 q.sync[AG_SYNC_COUNT] = 0;
                 q.sync[AG_SYNC_BIN] = 0;
+                q.sync[AG_SYNC_KEPT] = 0;
                 sh.gen = g;
                 asm volatile("fence.acq_rel.gpu;" ::: "memory");
                 asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(q.sync + AG_SYNC_GEN), "r"(g) : "memory");
@@ -475,11 +496,12 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
             ag_st_keep_f32(c_out32 + r, c, pol_last);
     }
 
-    /* the reference's per-vertex update for a finished row sum; data-driven
+    /* the reference's per-vertex update for a finished row sum (rank at `at`,
+     * device row r); data-driven
      * passes carry the row's tag in the sum's sign bit: rows off the worklist
      * and rows that moved by less than epsilon keep rank and contribution
      * (sign cleared, pageRank.c:2896-2916) */
-    __device__ __forceinline__ void finish(uint32_t r, float s, float rp, uint32_t od)
+    __device__ __forceinline__ void finish(uint32_t at, uint32_t r, float s, float rp, uint32_t od)
     {
         if (MODE == AG_MODE_DD) {
             if (iter == 0 || (__float_as_uint(s) >> 31)) {
@@ -487,7 +509,7 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
                 const double err = (double)fabsf(__fsub_rn(rn, rp));
                 my_err += err;
                 if (err >= eps) {
-                    p.rank[r] = rn;
+                    p.rank[at] = rn;
                     const float c = od ? __fdiv_rn(rn, __uint2float_rn(od)) : 0.0f;
                     ag_st_keep_f32(c_out32 + r, __uint_as_float(__float_as_uint(c) | 0x80000000u), pol_last);
                     ++my_active;
@@ -498,7 +520,7 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
             return;
         }
         const float rn = __fadd_rn(p.base, __fmul_rn(p.damp, s));
-        p.rank[r] = rn;
+        p.rank[at] = rn;
         const double err = (double)fabsf(__fsub_rn(rn, rp));
         my_err += err;
         my_active += (err >= eps) ? 1u : 0u;
@@ -613,7 +635,7 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
             const float s = sums[i];
             if (__float_as_uint(s) != AG_SV_HUB ||
                 __ldg(p.row_off + r0 + i + 1) - __ldg(p.row_off + r0 + i) <= AG_BIN_HUB)
-                finish(r0 + i, s, rp, od);
+                finish(r0 + i, r0 + i, s, rp, od);
             rp = rn;
             od = on;
         }
@@ -650,6 +672,39 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
         return lo;
     }
 
+    /* maps of a round from its values (eight per lane).  A round that should
+     * leave its binade (it did in the pass before) keeps the lanes' maps and
+     * values for the composer. */
+    __device__ __forceinline__ void map_round(const float *v, uint32_t pred, uint32_t next, uint4 *words)
+    {
+        const uint32_t lo = ag_sv_low_exp(pred, next);
+        uint32_t w0 = AG_XNOT, w1 = AG_XNOT, slot = AG_SV_NOT_KEPT;
+        if (lo >= 24u && lo < 254u) {
+            uint32_t a0, a1, b0, b1;
+            ag_sv_moves(v, lo, a0, a1);
+            ag_sv_moves(v, lo + 1u, b0, b1);
+            if ((next >> 7) > (pred >> 7)) {
+                if (lane == 0)
+                    slot = atomicAdd(q.sync + AG_SYNC_KEPT, 1u);
+                slot = __shfl_sync(0xffffffffu, slot, 0);
+                if (slot < q.kept_cap) {
+                    float4 *k = q.kept + (size_t)slot * AG_KEPT_QUADS;
+                    reinterpret_cast<uint4 *>(k)[lane] = make_uint4(a0, a1, b0, b1);
+                    k[32 + 2 * lane] = make_float4(v[0], v[1], v[2], v[3]);
+                    k[33 + 2 * lane] = make_float4(v[4], v[5], v[6], v[7]);
+                } else {
+                    slot = AG_SV_NOT_KEPT;
+                }
+            }
+            ag_sv_scan(lane, a0, a1);
+            ag_sv_scan(lane, b0, b1);
+            w0 = ag_sv_pack(a0, a1);
+            w1 = ag_sv_pack(b0, b1);
+        }
+        if (lane == 31)
+            *words = make_uint4(w0, w1, slot, 0u);
+    }
+
     /* ------------------------------------------------------------ hub bin */
     /* Chunks [c0, c0 + nc) of hub rows, staged together.  FAST: a warp sums
      * each chunk.  EXACT: the rounds of 256 values of a chunk are mapped by
@@ -660,8 +715,8 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
     {
         const uint32_t c0 = k * q.per_bin, nc = min(q.per_bin, q.nhub - c0);
         if (EXACT)
-            for (uint32_t i = st; i < nc * AG_BIN_ROUNDS; i += AG_SUB_THREADS)
-                sh.pred[sub][i] = *((volatile uint8_t *)(q.hub_pred + (size_t)c0 * AG_BIN_ROUNDS + i));
+            for (uint32_t i = st; i <= nc * AG_BIN_ROUNDS; i += AG_SUB_THREADS)
+                sh.pred[sub][i] = __ldcg(q.hub_pred + (size_t)c0 * AG_BIN_ROUNDS + i);
         stage(vals, q.ids + (size_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
         ag_sv_sub_sync(sub);
         if (EXACT) {
@@ -677,18 +732,10 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
                 }
                 if (rd * AG_BIN_ROUND >= len)
                     continue;
-                const uint32_t e = sh.pred[sub][t];
-                uint32_t word = AG_XNOT;
-                if (e >= 24u && e <= 254u) {
-                    float v[8];
-                    uint32_t d0, d1;
-                    ag_sv_eight<MODE>(v0 + rd * AG_BIN_ROUND, len - rd * AG_BIN_ROUND, lane, v);
-                    ag_sv_moves(v, e, d0, d1);
-                    ag_sv_scan(lane, d0, d1);
-                    word = ag_sv_pack(d0, d1);
-                }
-                if (lane == 31)
-                    q.hub_words[(size_t)c0 * AG_BIN_ROUNDS + t] = word;
+                float v[8];
+                ag_sv_eight<MODE>(v0 + rd * AG_BIN_ROUND, len - rd * AG_BIN_ROUND, lane, v);
+                const size_t k = (size_t)c0 * AG_BIN_ROUNDS + t;
+                map_round(v, sh.pred[sub][t], sh.pred[sub][t + 1], q.hub_words + k);
             }
             ag_sv_sub_sync(sub);
         }
@@ -733,7 +780,7 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
             __threadfence();
             float s;
             if (EXACT) {
-                s = compose(h, v0);
+                s = compose(h);
             } else {
                 double t = 0.0;
                 for (uint32_t c = lane; c < nch; c += 32)
@@ -746,7 +793,7 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
                 q.hub_seen[h.z] = 0;
                 const uint32_t r = h.x;
                 if (MODE != AG_MODE_MULTI || !*((volatile uint32_t *)(p.g_done + graph_of(r))))
-                    finish(r, s, ag_ld_rank(p.rank + r), ag_ld_row_u32(p.outdeg + r));
+                    finish(r, r, s, ag_ld_rank(p.rank + r), ag_ld_row_u32(p.outdeg + r));
             }
             __syncwarp();
             if (MODE == AG_MODE_MULTI)
@@ -755,42 +802,49 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
         ag_sv_sub_sync(sub);
     }
 
-    /* EXACT order, on the warp of a hub row's last chunk: the row's rounds in
-     * order from its head sum, 32 words at a time.  Words whose exponent is
-     * s's compose (a scan of the lanes' maps); the first that does not apply
-     * is added value by value (ag_sv_round) from its gathered values, and the
-     * words after it go on.  Records each round's starting exponent.
-     * `vals`: 256 floats of the warp's own. */
-    __device__ float compose(const uint4 h, float *vals)
+    /* EXACT order: a hub row on one warp, its rounds in order from its head
+     * sum, 32 at a time.  Maps at s's exponent compose (a scan of the lanes'
+     * maps); the first that does not apply is added from its values
+     * (ag_sv_round), kept by the chunk or gathered again, and the rounds after
+     * it go on.  Records where each round began. */
+    __device__ float compose(const uint4 h)
     {
-        const uint32_t nch = h.w >> 11, total = nch * AG_BIN_ROUNDS;
         const uint32_t deg = __ldg(p.row_off + h.x + 1) - __ldg(p.row_off + h.x);
         const uint32_t rounds = (deg + AG_BIN_ROUND - 1u) / AG_BIN_ROUND;
-        const uint32_t *words = q.hub_words + (size_t)h.z * AG_BIN_ROUNDS;
-        uint8_t *pred = q.hub_pred + (size_t)h.z * AG_BIN_ROUNDS;
-        const uint32_t *ids = q.ids + (size_t)h.z * AG_BIN_HUB;
+        const size_t k0 = (size_t)h.z * AG_BIN_ROUNDS;
+        const uint4 *words = q.hub_words + k0;
+        uint16_t *pred = q.hub_pred + k0;
+        const uint4 *ids = reinterpret_cast<const uint4 *>(q.ids) + k0 * (AG_BIN_ROUND / 4);
         float s = (float)__ldcg(q.hub_sum + h.z);
-        uint32_t wn = lane < total ? __ldcg(words + lane) : 0u;
-        uint32_t en = lane < total ? *((volatile uint8_t *)(pred + lane)) : 0u;
+        uint4 wn = make_uint4(0, 0, 0, 0);
+        uint32_t en = 0, em = 0;
+        if (lane < rounds) {
+            wn = __ldcg(words + lane);
+            en = __ldcg(pred + lane);
+            em = __ldcg(pred + lane + 1);
+        }
         for (uint32_t b = 0; b < rounds; b += 32) {
-            const uint32_t w = wn, e = en, k = b + lane;
-            if (k + 32u < total) {
+            const uint4 w = wn;
+            const uint32_t lo = ag_sv_low_exp(en, em), k = b + lane;
+            uint32_t began = en;
+            if (k + 32u < rounds) {
                 wn = __ldcg(words + k + 32u);
-                en = *((volatile uint8_t *)(pred + k + 32u));
+                en = __ldcg(pred + k + 32u);
+                em = __ldcg(pred + k + 33u);
             }
             const bool live = k < rounds && k >= AG_BIN_HEAD / AG_BIN_ROUND;
-            uint32_t began = e; /* exponent where this lane's round began */
             uint32_t done = b ? 0u : AG_BIN_HEAD / AG_BIN_ROUND;
             while (done < 32u && b + done < rounds) {
                 const uint32_t sb = __float_as_uint(s), ex = sb >> 23;
                 const uint32_t m = (sb & 0x7fffffu) | 0x800000u;
                 uint32_t d0 = 0, d1 = 0;
                 if (live && lane >= done) {
-                    if ((w & AG_XNOT) || e != ex || ex < 24u || ex > 254u) {
+                    const uint32_t x = ex == lo ? w.x : ex == lo + 1u ? w.y : AG_XNOT;
+                    if ((x & AG_XNOT) || ex < 24u || ex > 254u) {
                         d0 = d1 = 1u << 24;
                     } else {
-                        d0 = w & 0x3ffffffu;
-                        d1 = d0 + ((w >> 26) & 3u) - 1u;
+                        d0 = x & 0x3ffffffu;
+                        d1 = d0 + ((x >> 26) & 3u) - 1u;
                     }
                 }
                 ag_sv_scan(lane, d0, d1);
@@ -798,34 +852,74 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
                 const uint32_t ok = __ballot_sync(0xffffffffu, to < (1u << 24));
                 const uint32_t out = ok == 0xffffffffu ? 32u : __ffs(~ok) - 1;
                 const uint32_t before = __shfl_sync(0xffffffffu, to, (out - 1u) & 31u);
-                if (out > done) {
+                const uint32_t prev = __shfl_up_sync(0xffffffffu, to, 1);
+                if (lane >= done && lane <= out)
+                    began = (ex << 7) | (((lane > done ? prev : m) >> 16) & 0x7fu);
+                if (out > done)
                     s = ag_sv_make(ex, before);
-                    if (lane >= done && lane < out)
-                        began = ex;
-                }
                 done = out;
                 if (out == 32u)
                     break;
-                /* this round's values, in stream order */
-                if (lane == out)
-                    began = __float_as_uint(s) >> 23;
-                const uint32_t r0 = (b + out) * AG_BIN_ROUND, n = min(AG_BIN_ROUND, deg - r0);
-                uint32_t u[8];
+                /* this round from its values, eight consecutive ones per lane */
+                const uint32_t r = b + out, slot = __shfl_sync(0xffffffffu, w.z, out);
+                const uint32_t e0 = __shfl_sync(0xffffffffu, lo, out);
+                float v[8];
+                uint32_t from = 0;
+                if (slot != AG_SV_NOT_KEPT) {
+                    const float4 *kp = q.kept + (size_t)slot * AG_KEPT_QUADS;
+                    const uint4 mp = __ldcg(reinterpret_cast<const uint4 *>(kp) + lane);
+                    const float4 x = __ldcg(kp + 32 + 2 * lane), y = __ldcg(kp + 33 + 2 * lane);
+                    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+                    v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+                    if ((__float_as_uint(s) >> 23) == e0) {
+                        /* the lanes' maps below the binade's end, the lane that
+                         * leaves it value by value, the others' maps above it */
+                        from = mapped(mp.x, mp.y, v, 0u, s);
+                        if (from < 32u && (__float_as_uint(s) >> 23) == e0 + 1u)
+                            from = mapped(mp.z, mp.w, v, from, s);
+                    }
+                } else {
+                    const uint4 x = __ldg(ids + (size_t)r * (AG_BIN_ROUND / 4) + 2 * lane);
+                    const uint4 y = __ldg(ids + (size_t)r * (AG_BIN_ROUND / 4) + 2 * lane + 1);
+                    gather8(x, y, r * AG_BIN_ROUND + 8u * lane, deg, v);
+                    if (MODE == AG_MODE_DD)
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    u[i] = __ldg(ids + r0 + lane + 32 * i); /* padding ids are 0 */
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    vals[lane + 32 * i] = gather(u[i]);
-                __syncwarp();
-                s = ag_sv_round<MODE>(vals, n, s, lane);
+                        for (int i = 0; i < 8; ++i)
+                            v[i] = fabsf(v[i]);
+                }
+                if (from < 32u)
+                    s = ag_sv_round(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], s, lane, from);
                 done = out + 1u;
             }
             if (live)
-                pred[k] = (uint8_t)min(began, 255u);
+                pred[k] = (uint16_t)min(began, 0x7fffu);
         }
         return s;
+    }
+
+    /* lanes from `done` on move s by their maps (at s's exponent); the lane
+     * where s would leave its binade adds its values v.  Returns the lanes
+     * that are in s. */
+    __device__ __forceinline__ uint32_t mapped(uint32_t d0, uint32_t d1, const float *v, uint32_t done, float &s) const
+    {
+        const uint32_t sb = __float_as_uint(s), ex = sb >> 23, m = (sb & 0x7fffffu) | 0x800000u;
+        if (lane < done)
+            d0 = d1 = 0;
+        ag_sv_scan(lane, d0, d1);
+        const uint32_t to = m + ((m & 1u) ? d1 : d0);
+        const uint32_t ok = __ballot_sync(0xffffffffu, to < (1u << 24));
+        if (ok == 0xffffffffu) {
+            s = ag_sv_make(ex, __shfl_sync(0xffffffffu, to, 31));
+            return 32u;
+        }
+        const uint32_t out = __ffs(~ok) - 1;
+        const uint32_t before = __shfl_sync(0xffffffffu, to, (out - 1u) & 31u);
+        s = ag_sv_make(ex, out ? before : m);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            s = __fadd_rn(s, v[i]);
+        s = __shfl_sync(0xffffffffu, s, out);
+        return out + 1u;
     }
 
     /* EXACT order, before the first pass: each round's starting exponent from
@@ -852,10 +946,15 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
                 for (int o = 16; o > 0; o >>= 1)
                     x += __shfl_xor_sync(0xffffffffu, x, o);
                 if (lane == 0)
-                    q.hub_words[(size_t)c0 * AG_BIN_ROUNDS + t] = __float_as_uint(x);
+                    q.hub_words[(size_t)c0 * AG_BIN_ROUNDS + t].x = __float_as_uint(x);
             }
             ag_sv_sub_sync(sub);
         }
+        return predict_scan();
+    }
+
+    __device__ __forceinline__ bool predict_scan()
+    {
         const uint32_t f = flags;
         if (!grid_sync([&] { return f; }))
             return false;
@@ -868,7 +967,8 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
             float run = 0.0f;
             for (uint32_t b = 0; b < total; b += 32) {
                 const uint32_t k = b + lane;
-                const float x = k < total ? __uint_as_float(__ldcg(q.hub_words + (size_t)c * AG_BIN_ROUNDS + k)) : 0.0f;
+                const float x =
+                    k < total ? __uint_as_float(__ldcg(&q.hub_words[(size_t)c * AG_BIN_ROUNDS + k].x)) : 0.0f;
                 float inc = x;
 #pragma unroll
                 for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -878,11 +978,390 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
                 }
                 if (k < total)
                     q.hub_pred[(size_t)c * AG_BIN_ROUNDS + k] =
-                        (uint8_t)((__float_as_uint(run + (inc - x)) >> 23) & 0xffu);
+                        (uint16_t)(__float_as_uint(run + (inc - x)) >> 16);
                 run += __shfl_sync(0xffffffffu, inc, 31);
             }
         }
         return grid_sync([&] { return f; });
+    }
+
+    /* -------------------------------------------------------------- units */
+    /* eight gathered values of a lane's two quads; those at or past n are -0
+     * (s + -0 = s) */
+    __device__ __forceinline__ void gather8(const uint4 &a, const uint4 &b, uint32_t j, uint32_t n, float *v) const
+    {
+        v[0] = gather(a.x);
+        v[1] = gather(a.y);
+        v[2] = gather(a.z);
+        v[3] = gather(a.w);
+        v[4] = gather(b.x);
+        v[5] = gather(b.y);
+        v[6] = gather(b.z);
+        v[7] = gather(b.w);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (j + i >= n)
+                v[i] = -0.0f;
+    }
+
+    /* a lane's running sum over eight more values of its row of n in-edges */
+    struct RowSum
+    {
+        float s;      /* stream order                                          */
+        double t;     /* FAST order, rows above AG_BIN_SEQ in-edges            */
+        uint32_t neg; /* data-driven: sign bits                                */
+    };
+
+    __device__ __forceinline__ void add8(RowSum &a, float *v, uint32_t n) const
+    {
+        if (MODE == AG_MODE_DD) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                /* -0 past the end is no tag: its other bits are 0 */
+                a.neg |= v[i] != 0.0f ? __float_as_uint(v[i]) : 0u;
+                v[i] = fabsf(v[i]);
+            }
+        }
+        if (!EXACT && n > AG_BIN_SEQ) {
+            a.t += (double)__fadd_rn(__fadd_rn(__fadd_rn(v[0], v[1]), __fadd_rn(v[2], v[3])),
+                                     __fadd_rn(__fadd_rn(v[4], v[5]), __fadd_rn(v[6], v[7])));
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            a.s = __fadd_rn(a.s, v[i]);
+    }
+
+    __device__ __forceinline__ void unit_finish(uint32_t u, uint32_t info, const RowSum &sum, float rp, uint32_t od)
+    {
+        const uint32_t at = 32u * u + lane, n = AG_UNIT_LEN(info);
+        if (at >= p.N || (info & AG_UNIT_HUB))
+            return;
+        float s = n ? sum.s : 0.0f;
+        if (!EXACT && n > AG_BIN_SEQ)
+            s = __double2float_rn(sum.t);
+        if (MODE == AG_MODE_DD)
+            s = __uint_as_float((__float_as_uint(s) & 0x7fffffffu) | (sum.neg & 0x80000000u));
+        finish(at, (at & ~(AG_UNIT_WIN - 1u)) + AG_UNIT_ROW(info), s, rp, od);
+    }
+
+    /* the units with the longest rows, one after another */
+    __device__ __forceinline__ void heavy_unit(uint32_t u)
+    {
+        const uint32_t b0 = __ldg(q.ubaseq + u), rounds = (__ldg(q.ubaseq + u + 1) - b0) >> 5;
+        uint32_t info = 0, od = 0;
+        float rp = 0.0f;
+        unit_row(u, info, rp, od);
+        const uint32_t n = AG_UNIT_LEN(info);
+        uint4 a = make_uint4(0, 0, 0, 0), b = a;
+        pair(b0, rounds, a, b);
+        RowSum sum = {-0.0f, 0.0, 0u};
+        for (uint32_t i = 0; i < rounds; i += 2) {
+            uint4 na = make_uint4(0, 0, 0, 0), nb = na;
+            if (i + 2 < rounds)
+                pair(b0 + 32u * (i + 2), rounds - i - 2, na, nb);
+            float v[8];
+            gather8(a, b, 4u * i, n, v);
+            add8(sum, v, n);
+            a = na;
+            b = nb;
+        }
+        unit_finish(u, info, sum, rp, od);
+    }
+
+    /* the other units, a batch of consecutive ones at a time from an atomic
+     * counter (batch bt first, then those of the tickets drawn, first_ticket
+     * added modulo 2^32).  The next quads (of this unit or the next one) are on their way
+     * while a lane's eight gathers travel, and the next batch is drawn one
+     * batch ahead. */
+    __device__ __forceinline__ void units(uint32_t bt, uint32_t first_ticket)
+    {
+        if (bt >= q.nbatch)
+            return;
+        uint32_t u = __ldg(q.bstart + bt), end = __ldg(q.bstart + bt + 1);
+        uint32_t un = u, unn;         /* the next unit, the one after it */
+        uint32_t start_n = 0, end_n = 0;
+        uint32_t ticket = 0; /* lane 0: of the batch after the next one */
+        auto draw = [&]() {
+            bt = __shfl_sync(0xffffffffu, ticket, 0) + first_ticket;
+            start_n = end_n = q.nunits;
+            if (bt < q.nbatch) {
+                start_n = __ldg(q.bstart + bt);
+                end_n = __ldg(q.bstart + bt + 1);
+                if (lane == 0)
+                    ticket = atomicAdd(q.sync + AG_SYNC_BIN, 1u);
+            }
+        };
+        /* the unit after x in this warp's batches */
+        auto after = [&](uint32_t x) {
+            ++x;
+            while (x >= end && x < q.nunits) {
+                x = start_n;
+                end = end_n;
+                draw();
+            }
+            return x;
+        };
+        if (lane == 0)
+            ticket = atomicAdd(q.sync + AG_SYNC_BIN, 1u);
+        draw();
+        if (u >= end) /* an empty batch */
+            u = after(u - 1u);
+        if (u >= q.nunits)
+            return;
+        un = after(u);
+        uint32_t b0, rounds, info = 0, od = 0, bn, rn;
+        float rp = 0.0f;
+        unit_base(u, b0, rounds);
+        unit_base(un, bn, rn);
+        unit_row(u, info, rp, od);
+        uint4 a = make_uint4(0, 0, 0, 0), b = a;
+        pair(b0, rounds <= q.heavy_quads ? rounds : 0u, a, b);
+        for (;;) {
+            uint32_t info_n = 0, od_n = 0, bnn = 0, rnn = 0;
+            float rp_n = 0.0f;
+            unn = un;
+            if (un < q.nunits) {
+                unit_row(un, info_n, rp_n, od_n);
+                unn = after(un); /* q.nunits once they are used up */
+                unit_base(unn, bnn, rnn);
+            }
+            const uint32_t n = AG_UNIT_LEN(info), first_n = rn <= q.heavy_quads ? rn : 0u;
+            if (rounds <= q.heavy_quads) {
+                RowSum sum = {-0.0f, 0.0, 0u};
+                for (uint32_t i = 0; i < rounds; i += 2) {
+                    uint4 na = make_uint4(0, 0, 0, 0), nb = na;
+                    if (i + 2 < rounds)
+                        pair(b0 + 32u * (i + 2), rounds - i - 2, na, nb);
+                    else
+                        pair(bn, first_n, na, nb);
+                    float v[8];
+                    gather8(a, b, 4u * i, n, v);
+                    add8(sum, v, n);
+                    a = na;
+                    b = nb;
+                }
+                unit_finish(u, info, sum, rp, od);
+            }
+            if (rounds == 0 || rounds > q.heavy_quads)
+                pair(bn, first_n, a, b);
+            if (un >= q.nunits)
+                return;
+            u = un;
+            b0 = bn;
+            rounds = rn;
+            un = unn;
+            bn = bnn;
+            rn = rnn;
+            info = info_n;
+            rp = rp_n;
+            od = od_n;
+        }
+    }
+
+    __device__ __forceinline__ void unit_base(uint32_t u, uint32_t &b0, uint32_t &rounds) const
+    {
+        b0 = rounds = 0;
+        if (u < q.nunits) {
+            b0 = __ldg(q.ubaseq + u);
+            rounds = (__ldg(q.ubaseq + u + 1) - b0) >> 5;
+        }
+    }
+
+    __device__ __forceinline__ void unit_row(uint32_t u, uint32_t &info, float &rp, uint32_t &od) const
+    {
+        const uint32_t at = 32u * u + lane;
+        if (at < p.N) {
+            info = ag_ld_row_u32(q.info + at);
+            rp = ag_ld_rank(p.rank + at);
+            od = ag_ld_row_u32(q.uoutdeg + at);
+        }
+    }
+
+    /* this lane's quads at b0 and b0 + 32, as far as `left` rounds go */
+    __device__ __forceinline__ void pair(uint32_t b0, uint32_t left, uint4 &a, uint4 &b) const
+    {
+        if (left > 0)
+            a = ag_ld_stream_u4(q.uids + b0 + lane, pol_first);
+        if (left > 1)
+            b = ag_ld_stream_u4(q.uids + b0 + 32u + lane, pol_first);
+    }
+
+    /* EXACT order: the first AG_BIN_HEAD values of 32 hub rows, one row per lane */
+    __device__ __forceinline__ void heads(uint32_t k)
+    {
+        const uint32_t i = 32u * k + lane;
+        if (i >= q.nhrow)
+            return;
+        const uint32_t first = __ldg(q.hrow + i);
+        const uint4 *src = reinterpret_cast<const uint4 *>(q.ids) + (size_t)first * (AG_BIN_HUB / 4);
+        RowSum sum = {-0.0f, 0.0, 0u};
+        uint4 a = ag_ld_stream_u4(src, pol_first), b = ag_ld_stream_u4(src + 1, pol_first);
+        for (uint32_t j = 0; j < AG_BIN_HEAD; j += 8) {
+            uint4 na = a, nb = b;
+            if (j + 8 < AG_BIN_HEAD) {
+                na = ag_ld_stream_u4(src + j / 4 + 2, pol_first);
+                nb = ag_ld_stream_u4(src + j / 4 + 3, pol_first);
+            }
+            float v[8];
+            gather8(a, b, j, AG_BIN_HEAD, v);
+            add8(sum, v, 0);
+            a = na;
+            b = nb;
+        }
+        q.hub_sum[first] = (double)sum.s;
+        if (MODE == AG_MODE_DD)
+            q.hub_tag[first] = sum.neg >> 31;
+    }
+
+    /* a hub chunk on one warp, a lane's eight values of a round in registers;
+     * FAST: its sum; EXACT: its rounds' maps (predict: their plain sums) */
+    template <bool PREDICT> __device__ __forceinline__ void chunk(uint32_t c)
+    {
+        const uint4 h = __ldg(q.hubs + c);
+        const uint32_t len = (h.w & (AG_BIN_HUB - 1u)) + 1u;
+        const uint32_t rounds = (len + AG_BIN_ROUND - 1u) / AG_BIN_ROUND;
+        const bool head = EXACT && !PREDICT && h.y == 0;
+        const uint4 *src = reinterpret_cast<const uint4 *>(q.ids) + (size_t)c * (AG_BIN_HUB / 4) + 2u * lane;
+        uint32_t rd = head ? AG_BIN_HEAD / AG_BIN_ROUND : 0u;
+        uint32_t pred = 0, next = 0;
+        if (EXACT && !PREDICT && rd < rounds) {
+            pred = __ldcg(q.hub_pred + (size_t)c * AG_BIN_ROUNDS + rd);
+            next = __ldcg(q.hub_pred + (size_t)c * AG_BIN_ROUNDS + rd + 1);
+        }
+        uint4 a = make_uint4(0, 0, 0, 0), b = a;
+        if (rd < rounds) {
+            a = ag_ld_stream_u4(src + rd * (AG_BIN_ROUND / 4), pol_first);
+            b = ag_ld_stream_u4(src + rd * (AG_BIN_ROUND / 4) + 1, pol_first);
+        }
+        double t = 0.0;
+        uint32_t neg = 0;
+        for (; rd < rounds; ++rd) {
+            uint4 na = a, nb = b;
+            uint32_t after = 0;
+            if (EXACT && !PREDICT)
+                after = __ldcg(q.hub_pred + (size_t)c * AG_BIN_ROUNDS + rd + 2);
+            if (rd + 1 < rounds) {
+                na = ag_ld_stream_u4(src + (rd + 1) * (AG_BIN_ROUND / 4), pol_first);
+                nb = ag_ld_stream_u4(src + (rd + 1) * (AG_BIN_ROUND / 4) + 1, pol_first);
+            }
+            float v[8];
+            gather8(a, b, rd * AG_BIN_ROUND + 8u * lane, len, v);
+            if (MODE == AG_MODE_DD) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    neg |= v[i] != 0.0f ? __float_as_uint(v[i]) : 0u;
+                    v[i] = fabsf(v[i]);
+                }
+            }
+            if (PREDICT) {
+                float x = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    x += __shfl_xor_sync(0xffffffffu, x, o);
+                if (lane == 0)
+                    q.hub_words[(size_t)c * AG_BIN_ROUNDS + rd].x = __float_as_uint(x);
+            } else if (EXACT) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    v[i] = __fadd_rn(v[i], 0.0f); /* past the end: +0 */
+                const size_t k = (size_t)c * AG_BIN_ROUNDS + rd;
+                map_round(v, pred, next, q.hub_words + k);
+                pred = next;
+                next = after;
+            } else {
+                t += (double)__fadd_rn(__fadd_rn(__fadd_rn(v[0], v[1]), __fadd_rn(v[2], v[3])),
+                                       __fadd_rn(__fadd_rn(v[4], v[5]), __fadd_rn(v[6], v[7])));
+            }
+            a = na;
+            b = nb;
+        }
+        if (PREDICT) {
+            if (lane >= rounds && lane < AG_BIN_ROUNDS)
+                q.hub_words[(size_t)c * AG_BIN_ROUNDS + lane].x = 0u;
+            return;
+        }
+        if (!EXACT) {
+            t = ag_sv_warp_d(t);
+            if (lane == 0)
+                q.hub_sum[c] = t;
+        }
+        if (MODE == AG_MODE_DD) {
+            neg = __any_sync(0xffffffffu, neg >> 31) ? 1u : 0u;
+            /* a row's first chunk shares its tag with its head */
+            if (lane == 0)
+                q.hub_tag[head ? q.nhub + c : c] = neg;
+        }
+    }
+
+    /* the hub rows from their chunks, a warp each (a grid barrier before it) */
+    __device__ __forceinline__ void hub_rows()
+    {
+        for (uint32_t i = (tid >> 5) * gridDim.x + blockIdx.x; i < q.nhrow; i += gridDim.x * (AG_SOLVE_BLK / 32)) {
+            const uint4 h = __ldg(q.hubs + __ldg(q.hrow + i));
+            const uint32_t at = __ldg(q.posof + h.x), nch = h.w >> 11;
+            float rp = 0.0f;
+            uint32_t od = 0, tag = 0;
+            if (lane == 0) {
+                rp = ag_ld_rank(p.rank + at);
+                od = ag_ld_row_u32(q.uoutdeg + at);
+            }
+            if (MODE == AG_MODE_DD) {
+                for (uint32_t c = lane; c < nch; c += 32)
+                    tag |= __ldcg(q.hub_tag + h.z + c);
+                if (EXACT)
+                    tag |= __ldcg(q.hub_tag + q.nhub + h.z);
+            }
+            float s;
+            if (EXACT) {
+                s = compose(h);
+            } else {
+                double t = 0.0;
+                for (uint32_t c = lane; c < nch; c += 32)
+                    t += __ldcg(q.hub_sum + h.z + c);
+                s = __double2float_rn(ag_sv_warp_d(t));
+            }
+            if (MODE == AG_MODE_DD && __any_sync(0xffffffffu, tag))
+                s = __uint_as_float(__float_as_uint(s) | 0x80000000u);
+            if (lane == 0)
+                finish(at, h.x, s, rp, od);
+        }
+    }
+
+    /* every unit and hub chunk of a pass, long chains first */
+    __device__ __forceinline__ bool unit_pass()
+    {
+        const uint32_t w = (tid >> 5) * gridDim.x + blockIdx.x, nw = gridDim.x * (AG_SOLVE_BLK / 32);
+        if (EXACT && iter == 0 && q.nhub) {
+            for (uint32_t c = w; c < q.nhub; c += nw)
+                chunk<true>(c);
+            if (!predict_scan())
+                return false;
+        }
+        const uint32_t nheads = EXACT ? (q.nhrow + 31u) / 32u : 0u;
+        /* items longest first, the next one drawn while one runs */
+        const uint32_t nlong = nheads + q.nhub + q.nheavy;
+        uint32_t t = w;
+        while (t < nlong) {
+            uint32_t ticket = 0;
+            if (lane == 0)
+                ticket = atomicAdd(q.sync + AG_SYNC_BIN, 1u);
+            if (t < q.nheavy)
+                heavy_unit(__ldg(q.heavy + t));
+            else if (EXACT && t < q.nheavy + nheads)
+                heads(t - q.nheavy);
+            else
+                chunk<false>(t - q.nheavy - nheads);
+            t = __shfl_sync(0xffffffffu, ticket, 0) + nw;
+        }
+        units(t - nlong, nw - nlong);
+        if (q.nhub) {
+            const uint32_t f = flags;
+            if (!grid_sync([&] { return f; }))
+                return false;
+            hub_rows();
+        }
+        return true;
     }
 
     /* --------------------------------------------------------------- pass */
@@ -892,10 +1371,14 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
         const uint32_t nall = q.nhb + q.nbins;
         uint32_t k = blockIdx.x + sub * gridDim.x;
         wait_hot();
-        if (EXACT && iter == 0 && q.nhub)
+        if (UNITS) {
+            if (!unit_pass())
+                return false;
+        } else if (EXACT && iter == 0 && q.nhub) {
             if (!predict(vals))
                 return false;
-        while (k < nall) {
+        }
+        while (!UNITS && k < nall) {
             /* the next bin's ticket is drawn while this one runs */
             uint32_t ticket = 0;
             if (st == 0)
@@ -1030,7 +1513,7 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
         for (uint64_t v = t0; v < p.N; v += n) {
             /* device row v is caller vertex perm[v]; the warm start is in caller order */
             const float r0 = run.use_init ? p.init_ranks[p.perm ? p.perm[v] : v] : p.base;
-            p.rank[v] = r0;
+            p.rank[UNITS ? q.posof[v] : (uint32_t)v] = r0;
             const uint32_t od = p.outdeg[v];
             const float c = od ? __fdiv_rn(r0, __uint2float_rn(od)) : 0.0f;
             if (PREC != 0)
@@ -1081,8 +1564,16 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
                 const uint32_t g = graph_of((uint32_t)v);
                 div = __uint2float_rn(__ldg(p.gstart + g + 1) - __ldg(p.gstart + g));
             }
-            const float r = __fdiv_rn(ag_ld_rank(p.rank + (p.inv ? p.inv[v] : v)), div);
-            p.out[v] = r;
+            /* caller vertex v, or the vertex of position v */
+            uint32_t at = (uint32_t)v, to = (uint32_t)v;
+            if (UNITS) {
+                to = (at & ~(AG_UNIT_WIN - 1u)) + AG_UNIT_ROW(q.info[at]);
+                to = p.perm ? p.perm[to] : to;
+            } else if (p.inv) {
+                at = p.inv[v];
+            }
+            const float r = __fdiv_rn(ag_ld_rank(p.rank + at), div);
+            p.out[to] = r;
             sum += (double)r;
         }
         sum = ag_sv_warp_d(sum);
@@ -1097,11 +1588,11 @@ template <int MODE, int PREC, bool EXACT> struct AgSolve
     }
 };
 
-template <int MODE, int PREC, bool EXACT>
+template <int MODE, int PREC, bool EXACT, bool UNITS>
 __global__ void __launch_bounds__(AG_SOLVE_BLK, 1) ag_solve_kernel(const AgSolveParams q, const AgRunConfig run)
 {
     __shared__ AgSvShared sh;
-    AgSolve<MODE, PREC, EXACT> s(q, sh);
+    AgSolve<MODE, PREC, EXACT, UNITS> s(q, sh);
     float *vals = reinterpret_cast<float *>(ag_sv_dyn + (size_t)q.p.hot_n * 4) + (size_t)s.sub * q.buf;
     if (threadIdx.x == 0)
         ag_sv_mbar_init(&sh.mbar);
@@ -1128,18 +1619,23 @@ __global__ void __launch_bounds__(AG_SOLVE_BLK, 1) ag_solve_kernel(const AgSolve
         s.normalise();
 }
 
-template <int MODE, int PREC> static const void *solve_ptr(int exact)
+template <int MODE, int PREC, bool UNITS> static const void *solve_ptr(int exact)
 {
-    return exact ? (const void *)ag_solve_kernel<MODE, PREC, true> : (const void *)ag_solve_kernel<MODE, PREC, false>;
+    return exact ? (const void *)ag_solve_kernel<MODE, PREC, true, UNITS>
+                 : (const void *)ag_solve_kernel<MODE, PREC, false, UNITS>;
 }
 
-extern "C" const void *ag_solve_kernel_ptr(int mode, int prec, int exact)
+extern "C" const void *ag_solve_kernel_ptr(int mode, int prec, int exact, int units)
 {
     if (mode == AG_MODE_MULTI)
-        return solve_ptr<AG_MODE_MULTI, 0>(exact);
+        return solve_ptr<AG_MODE_MULTI, 0, false>(exact);
     if (mode == AG_MODE_DD)
-        return solve_ptr<AG_MODE_DD, 0>(exact);
-    return prec == 1 ? solve_ptr<AG_MODE_PR, 1>(exact)
-           : prec == 2 ? solve_ptr<AG_MODE_PR, 2>(exact)
-                       : solve_ptr<AG_MODE_PR, 0>(exact);
+        return units ? solve_ptr<AG_MODE_DD, 0, true>(exact) : solve_ptr<AG_MODE_DD, 0, false>(exact);
+    if (units)
+        return prec == 1   ? solve_ptr<AG_MODE_PR, 1, true>(exact)
+               : prec == 2 ? solve_ptr<AG_MODE_PR, 2, true>(exact)
+                           : solve_ptr<AG_MODE_PR, 0, true>(exact);
+    return prec == 1   ? solve_ptr<AG_MODE_PR, 1, false>(exact)
+           : prec == 2 ? solve_ptr<AG_MODE_PR, 2, false>(exact)
+                       : solve_ptr<AG_MODE_PR, 0, false>(exact);
 }

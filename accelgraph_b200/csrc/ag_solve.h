@@ -4,7 +4,7 @@
 #ifndef AG_SOLVE_H
 #define AG_SOLVE_H
 
-#include "ag_bins.h"
+#include "ag_units.h"
 #include "ag_device.h"
 
 #ifndef AG_SUBS
@@ -18,7 +18,9 @@
 #define AG_SYNC_COUNT 0       /* CTAs that have arrived                         */
 #define AG_SYNC_GEN 1         /* barriers passed << 3 | flags                   */
 #define AG_SYNC_BIN 2         /* bins handed out in this pass                   */
+#define AG_SYNC_KEPT 3        /* rounds kept in this pass                       */
 #define AG_SYNC_WORDS 4
+#define AG_KEPT_QUADS 96u     /* 16-byte words of a kept round                  */
 #define AG_GEN_STOP 1u
 #define AG_GEN_READ_LOW 2u
 #define AG_GEN_WRITE_LOW 4u
@@ -32,10 +34,21 @@ typedef struct AgSolveParams
     uint32_t nbins, nhub;     /* row bins, hub chunks                           */
     uint32_t per_bin, nhb;    /* hub chunks per bin, bins they make             */
     uint32_t buf;             /* floats of a group's buffer                     */
+    /* units (nunits 0: bins): ids, hubs, nhub and the hub_* arrays are theirs */
+    uint32_t nunits, nhrow, nheavy, heavy_quads, nbatch;
+    const uint32_t *heavy, *bstart;
+    const uint32_t *info, *uoutdeg, *posof, *hrow;
+    const uint32_t *ubaseq;   /* AgUnitPlan::ubase                              */
+    const uint4 *uids;        /* the units' quads                               */
     double *hub_sum;          /* per chunk: FAST partial sum, EXACT head sum    */
-    uint32_t *hub_words;      /* EXACT: AG_BIN_ROUNDS words per chunk           */
-    uint8_t *hub_pred;        /* EXACT: biased exponent at each round's start   */
-    uint32_t *hub_seen;       /* per chunk (used at a row's first): chunks done */
+    uint4 *hub_words;         /* EXACT: per round its two maps and where its
+                                 values are kept                                */
+    uint16_t *hub_pred;       /* EXACT: the sum at each round's start, top half */
+    float4 *kept;             /* EXACT: lanes' maps (512 bytes) and values (1 KB)
+                                 of the rounds that should leave a binade       */
+    uint32_t kept_cap;        /* rounds it can hold                             */
+    uint32_t *hub_seen;       /* bins, per chunk (at a row's first): chunks done      */
+    uint32_t *hub_tag;        /* units, data-driven: a sign was set; 2 x nhub    */
     uint32_t *sync;           /* AG_SYNC_WORDS                                  */
     uint32_t spins;           /* polls of a grid barrier before it gives up     */
     uint32_t do_init, do_norm, max_pass; /* parts of a solve in this launch     */
@@ -44,7 +57,7 @@ typedef struct AgSolveParams
 #ifdef __cplusplus
 extern "C" {
 #endif
-const void *ag_solve_kernel_ptr(int mode, int prec, int exact);
+const void *ag_solve_kernel_ptr(int mode, int prec, int exact, int units);
 #ifdef __cplusplus
 }
 #endif
