@@ -282,7 +282,7 @@ typedef struct AgPlanState
     const uint32_t *row_off, *gstart;
     uint32_t n, cap, whub, ngraphs, nseg;
     void *scratch;
-    uint32_t *scan;
+    uint4 *scan;
 } AgPlanState;
 
 /* forward and inverse CSR in device memory, caller vertex order (ag_build.cu) */
@@ -308,6 +308,10 @@ extern "C" {
  * returns cudaErrorInvalidValue with *bad_edge = its lowest edge index */
 cudaError_t ag_csr_build_device(uint32_t n, uint32_t m, const uint32_t *src, const uint32_t *dst, const float *w,
                                 uint32_t flags, AgDevCSR *out, uint32_t *bad_edge, cudaStream_t s);
+/* the inverse CSR and out-degrees alone, sorted (AG_BUILD_SORT or, with
+ * dedupe, AG_BUILD_DEDUPE); errors as above */
+cudaError_t ag_inverse_build_device(uint32_t n, uint32_t m, const uint32_t *src, const uint32_t *dst, const float *w,
+                                    int dedupe, AgDevCSR *out, uint32_t *bad_edge, cudaStream_t s);
 void ag_csr_free_device(AgDevCSR *c, cudaStream_t s);
 
 

@@ -57,8 +57,17 @@ __global__ void ag_permuted_degrees_kernel(const uint32_t *perm, const uint32_t 
  * (coalesced stores) over a window of 32 consecutive rows: each lane holds
  * one row's old start and new start, and a position's row is found by a
  * five-step binary search over the lanes (shuffles).  When the window's rows
- * end before the segment does, the window moves on. */
-#define AG_COPY_SEG 2048u
+ * end before the segment does, the window moves on.  Bound by the latency of
+ * the id and its mapped id: AG_COPY_DEEP positions per lane are in flight, and
+ * short segments give every SM its warps (one position and 2048 in-edges a
+ * segment: 571 us at 1 M vertices and 16 M in-edges, 244 at 65 K and 1 M; now
+ * 298 and 108). */
+#ifndef AG_COPY_SEG
+#define AG_COPY_SEG 512u
+#endif
+#ifndef AG_COPY_DEEP
+#define AG_COPY_DEEP 4u
+#endif
 
 __global__ void ag_copy_rows_kernel(const uint32_t *perm, const uint32_t *inv, const uint32_t *off_old,
                                     const uint32_t *off_new, const uint32_t *ids_old, uint32_t *ids_new,
@@ -87,22 +96,34 @@ __global__ void ag_copy_rows_kernel(const uint32_t *perm, const uint32_t *inv, c
             const uint32_t src = i < n ? off_old[perm[i]] : 0u;
             const uint32_t wend = off_new[rbase + 32 < n ? rbase + 32 : n];
             const uint32_t stop = min(p1, wend);
-            for (; jb < stop; jb += 32) {
-                const uint32_t j = jb + lane;
-                /* the last lane whose row starts at or before j owns it (an
-                 * empty row shares its start with the next row, which wins) */
-                uint32_t l = 0;
+            for (; jb < stop; jb += 32 * AG_COPY_DEEP) {
+                /* AG_COPY_DEEP positions per lane, their loads in flight together */
+                uint32_t k[AG_COPY_DEEP], id[AG_COPY_DEEP];
 #pragma unroll
-                for (uint32_t step = 16; step >= 1; step >>= 1) {
-                    const uint32_t cand = l + step;
-                    if (__shfl_sync(0xffffffffu, dst, cand) <= j)
-                        l = cand;
+                for (uint32_t q = 0; q < AG_COPY_DEEP; ++q) {
+                    const uint32_t j = jb + 32 * q + lane;
+                    /* the last lane whose row starts at or before j owns it (an
+                     * empty row shares its start with the next row, which wins) */
+                    uint32_t l = 0;
+#pragma unroll
+                    for (uint32_t step = 16; step >= 1; step >>= 1) {
+                        const uint32_t cand = l + step;
+                        if (__shfl_sync(0xffffffffu, dst, cand) <= j)
+                            l = cand;
+                    }
+                    k[q] = __shfl_sync(0xffffffffu, src, l) + (j - __shfl_sync(0xffffffffu, dst, l));
                 }
-                const uint32_t k = __shfl_sync(0xffffffffu, src, l) + (j - __shfl_sync(0xffffffffu, dst, l));
-                if (j < stop) {
-                    ids_new[j] = inv[ids_old[k]];
-                    if (w_new)
-                        w_new[j] = w_old[k];
+#pragma unroll
+                for (uint32_t q = 0; q < AG_COPY_DEEP; ++q)
+                    id[q] = jb + 32 * q + lane < stop ? ids_old[k[q]] : 0u;
+#pragma unroll
+                for (uint32_t q = 0; q < AG_COPY_DEEP; ++q) {
+                    const uint32_t j = jb + 32 * q + lane;
+                    if (j < stop) {
+                        ids_new[j] = inv[id[q]];
+                        if (w_new)
+                            w_new[j] = w_old[k[q]];
+                    }
                 }
             }
             jb = stop;

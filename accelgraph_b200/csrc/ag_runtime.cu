@@ -2704,7 +2704,7 @@ static ag_status_t stage_in(const void *p, size_t bytes, const void **dev, void 
 }
 
 static ag_status_t build_device_csr(uint32_t N, uint64_t m, const uint32_t *src, const uint32_t *dst,
-                                    const float *w, uint32_t flags, AgDevCSR *csr)
+                                    const float *w, uint32_t flags, bool inverse_only, AgDevCSR *csr)
 {
     memset(csr, 0, sizeof(*csr));
     if (m > 0 && (!src || !dst))
@@ -2756,8 +2756,13 @@ static ag_status_t build_device_csr(uint32_t N, uint64_t m, const uint32_t *src,
     }
     if (st == AG_OK) {
         uint32_t bad = UINT32_MAX;
-        cudaError_t e = ag_csr_build_device(N, (uint32_t)m, (const uint32_t *)ds, (const uint32_t *)dd,
-                                            (const float *)dw, flags & ~AG_BUILD_SYMMETRIC, csr, &bad, s);
+        cudaError_t e;
+        if (inverse_only && (flags & (AG_BUILD_SORT | AG_BUILD_DEDUPE)))
+            e = ag_inverse_build_device(N, (uint32_t)m, (const uint32_t *)ds, (const uint32_t *)dd, (const float *)dw,
+                                        (flags & AG_BUILD_DEDUPE) != 0, csr, &bad, s);
+        else
+            e = ag_csr_build_device(N, (uint32_t)m, (const uint32_t *)ds, (const uint32_t *)dd, (const float *)dw,
+                                    flags & ~AG_BUILD_SYMMETRIC, csr, &bad, s);
         if (sym && bad != UINT32_MAX)
             bad = bad % (uint32_t)(m / 2); /* report the input edge */
         if (e != cudaSuccess) {
@@ -2785,7 +2790,7 @@ extern "C" struct GraphCSR *ag_graph_build_csr(uint32_t num_vertices, uint64_t n
 {
     ag_clear_error();
     AgDevCSR c;
-    if (build_device_csr(num_vertices, num_edges, src, dst, weight, flags, &c) != AG_OK)
+    if (build_device_csr(num_vertices, num_edges, src, dst, weight, flags, false, &c) != AG_OK)
         return nullptr;
     const uint32_t N = c.N, E = c.E;
     struct GraphCSR *g = ag_host_graph_new(N, E, weight != nullptr, (flags & AG_BUILD_PINNED) ? 1 : 0);
@@ -2827,7 +2832,7 @@ extern "C" ag_status_t ag_graph_build(uint32_t num_vertices, uint64_t num_edges,
         return ag_set_error(AG_ERR_INVALID_ARG, "ag_graph_build: NULL output");
     *out = nullptr;
     AgDevCSR c;
-    ag_status_t st = build_device_csr(num_vertices, num_edges, src, dst, weight, build_flags, &c);
+    ag_status_t st = build_device_csr(num_vertices, num_edges, src, dst, weight, build_flags, true, &c);
     if (st != AG_OK)
         return st;
     st = upload_impl(nullptr, upload_flags, nullptr, 0, 0, out, &c);

@@ -262,8 +262,20 @@ template <int MODE> __device__ __forceinline__ float ag_sv_fast(const float *val
 {
     const float4 *q = reinterpret_cast<const float4 *>(vals);
     auto mag = [](float x) { return MODE == AG_MODE_DD ? fabsf(x) : x; };
-    double t = 0.0;
-    for (uint32_t j = 0; j < n; j += 8u, q += 2) {
+    /* two sums, so that one eight's tree runs while the other is added */
+    double t = 0.0, t1 = 0.0;
+    auto eight = [&](float4 a, float4 b) {
+        const float x = __fadd_rn(__fadd_rn(mag(a.x), mag(a.y)), __fadd_rn(mag(a.z), mag(a.w)));
+        const float y = __fadd_rn(__fadd_rn(mag(b.x), mag(b.y)), __fadd_rn(mag(b.z), mag(b.w)));
+        return (double)__fadd_rn(x, y);
+    };
+    uint32_t j = 0;
+    for (; j + 16u <= n; j += 16u, q += 4) {
+        const float4 a = q[0], b = q[1], c = q[2], d = q[3];
+        t += eight(a, b);
+        t1 += eight(c, d);
+    }
+    for (; j < n; j += 8u, q += 2) {
         float4 a = q[0], b = q[1];
         if (j + 8u > n) {
             const uint32_t m = n - j; /* 1 .. 7 */
@@ -275,10 +287,9 @@ template <int MODE> __device__ __forceinline__ float ag_sv_fast(const float *val
             if (m < 7) b.z = 0.0f;
             b.w = 0.0f;
         }
-        const float x = __fadd_rn(__fadd_rn(mag(a.x), mag(a.y)), __fadd_rn(mag(a.z), mag(a.w)));
-        const float y = __fadd_rn(__fadd_rn(mag(b.x), mag(b.y)), __fadd_rn(mag(b.z), mag(b.w)));
-        t += (double)__fadd_rn(x, y);
+        t += eight(a, b);
     }
+    t += t1;
     return __double2float_rn(t);
 }
 

@@ -106,3 +106,26 @@ def test_device_graph_from_edges_pagerank(gpu, oracle):
     y_built = dg.spmv(x, ag.AG_SPMV_GRAPH_WEIGHTS | ag.AG_SPMV_EXACT)
     y_up = ag.DeviceGraph(host, weights=True).spmv(x, ag.AG_SPMV_GRAPH_WEIGHTS | ag.AG_SPMV_EXACT)
     assert np.array_equal(y_built, y_up)
+
+
+@pytest.mark.parametrize("n,m", [(1, 0), (1, 5), (7, 1), (300, 2047), (300, 2048), (300, 2049), (40, 9000), (70001, 50001)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_sorted_device_graph_matches_upload(gpu, n, m, weighted):
+    """The one-sort build of a sorted device graph against the uploaded host build: edges and work list equal, EXACT
+    ranks (out-degrees) and products (in-neighbours, weights of the first of equal edges) bit for bit."""
+    ag = gpu
+    rng = np.random.default_rng(n + m)
+    src, dst = rng.integers(0, n, m).astype(np.uint32), rng.integers(0, n, m).astype(np.uint32)
+    w = rng.random(m, dtype=np.float32) if weighted else None
+    for flags in (ag.AG_BUILD_SORT, ag.AG_BUILD_DEDUPE, ag.AG_BUILD_DEDUPE | ag.AG_BUILD_SYMMETRIC):
+        up = ag.DeviceGraph(ag.Graph.from_edges(n, src, dst, w, flags), weights=weighted)
+        dev = ag.DeviceGraph.from_edges(n, src, dst, w, build_flags=flags)
+        assert dev.num_edges == up.num_edges and np.array_equal(dev.tasks(), up.tasks())
+        a, b = (g.pagerank(10, 1e-6, order=ag.AG_ORDER_EXACT)[0] for g in (dev, up))
+        assert np.array_equal(a, b)
+        x = rng.random(n, dtype=np.float32)
+        assert np.array_equal(dev.spmv(x, ag.AG_SPMV_EXACT), up.spmv(x, ag.AG_SPMV_EXACT))
+    if m > 100:
+        src[77] = n
+        with pytest.raises(ag.AGError, match="edge 77 "):
+            ag.DeviceGraph.from_edges(n, src, dst, w)
