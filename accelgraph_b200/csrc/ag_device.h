@@ -162,6 +162,8 @@ typedef struct AgControl
     uint32_t stop;            /* 1 once the loop is over (stream launches)  */
     uint32_t fault;           /* nonzero: a bounded device wait ran out     */
     double last_err_sum;      /* sum of |r' - r| of the last closed pass    */
+    double last_err;          /* error total of the last closed pass        */
+    uint32_t last_active;     /* active vertices of the last closed pass    */
     uint32_t hist_active[AG_MAX_HISTORY];
     double hist_err[AG_MAX_HISTORY];
     unsigned long long hist_t[AG_MAX_HISTORY];
@@ -324,6 +326,10 @@ cudaError_t ag_plan_count(const uint32_t *row_off, uint32_t n, uint32_t cap, uin
 cudaError_t ag_plan_write(AgPlanState *ps, const uint32_t *totals, uint4 *fast, uint4 *exact, cudaStream_t s);
 void ag_plan_release(AgPlanState *ps, cudaStream_t s);
 cudaError_t ag_set_u32(uint32_t *p, uint32_t v, cudaStream_t s);
+
+/* copy device memory to host memory behind the library stream's work and wait
+ * for it (bounded) */
+int32_t ag_rt_copy_to_host(void *dst, const void *src, size_t bytes);
 
 struct ag_graph_s;
 int32_t ag_rt_graph_view(struct ag_graph_s *g, AgGraphView *v);

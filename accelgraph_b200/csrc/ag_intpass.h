@@ -218,6 +218,8 @@ __device__ __forceinline__ void ag_close_pass(const AgPullParams &p, double err,
         const bool conv = act == 0;
         c->prev_err = e;
         c->last_err_sum = vc->err_acc;
+        c->last_err = e;
+        c->last_active = act;
         c->iter = P + 1;
         c->converged = conv ? 1u : 0u;
         const bool cont = !conv && (P + 1 < vc->max_iter);

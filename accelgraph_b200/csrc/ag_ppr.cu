@@ -365,7 +365,9 @@ extern "C" ag_status_t ag_ppr_spmm(ag_graph_t g, const uint32_t *sources, uint32
         PCHK(cudaMallocAsync((void **)&out, (size_t)gv.N * k * sizeof(float), s));
         ag_ppr_output_kernel<<<ag_sm_grid(8), 256, 0, s>>>(p, gv.perm, out);
         PCHK(cudaGetLastError());
-        PCHK(cudaMemcpyAsync(ranks, out, (size_t)gv.N * k * sizeof(float), cudaMemcpyDeviceToHost, s));
+        st = ag_rt_copy_to_host(ranks, out, (size_t)gv.N * k * sizeof(float));
+        if (st != AG_OK)
+            goto done;
     }
     PCHK(cudaStreamSynchronize(s));
     cudaEventElapsedTime(&ms, e0, e1);
@@ -402,5 +404,5 @@ done:
         cudaGetLastError();
         return ag_set_error(AG_ERR_CUDA, "ag_ppr_spmm: %s", cudaGetErrorString(err));
     }
-    return AG_OK;
+    return st;
 }

@@ -1100,6 +1100,8 @@ __device__ __forceinline__ void ag_pull_body(const AgPullParams &p, double *s_re
         const bool conv = active == 0;
         c->prev_err = err;
         c->last_err_sum = vc->err_acc;
+        c->last_err = err;
+        c->last_active = active;
         c->iter = P + 1;
         c->converged = conv ? 1u : 0u;
         const bool cont = !conv && (P + 1 < vc->max_iter);

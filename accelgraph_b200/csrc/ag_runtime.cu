@@ -24,6 +24,7 @@
 #include <time.h>
 
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "ag_device.h"
@@ -139,25 +140,33 @@ static double wait_limit_s(double timeout_s)
     return 600.0;
 }
 
-/* bounded wait: poll the stream until it drains or the deadline passes */
-static ag_status_t stream_wait(cudaStream_t s, double timeout_s)
+/* Poll `query` until it succeeds or the deadline passes.  The first
+ * milliseconds are spun: a nap lasts about 70 us, a large part of a small
+ * solve (a 1 K-vertex solve of 150 us was collected 50 us late). */
+template <typename F> static ag_status_t poll_wait(F query, const char *what, double timeout_s)
 {
     const double limit = wait_limit_s(timeout_s);
     const double t0 = ag_wall_seconds();
-    unsigned spins = 0;
     for (;;) {
-        cudaError_t e = cudaStreamQuery(s);
+        cudaError_t e = query();
         if (e == cudaSuccess)
             return AG_OK;
         if (e != cudaErrorNotReady)
-            return ag_set_error(AG_ERR_CUDA, "stream failed: %s", cudaGetErrorString(e));
-        if (ag_wall_seconds() - t0 > limit)
-            return ag_set_error(AG_ERR_TIMEOUT, "device work did not finish within %.1f s", limit);
-        if (++spins > 64) {
+            return ag_set_error(AG_ERR_CUDA, "%s failed: %s", what, cudaGetErrorString(e));
+        const double t = ag_wall_seconds() - t0;
+        if (t > limit)
+            return ag_set_error(AG_ERR_TIMEOUT, "%s did not finish within %.1f s", what, limit);
+        if (t > 2e-3) {
             struct timespec ts = {0, 20000};
             nanosleep(&ts, nullptr);
         }
     }
+}
+
+/* bounded wait for the stream to drain */
+static ag_status_t stream_wait(cudaStream_t s, double timeout_s)
+{
+    return poll_wait([s] { return cudaStreamQuery(s); }, "device work", timeout_s);
 }
 
 extern "C" ag_status_t ag_synchronize(double timeout_s)
@@ -207,31 +216,47 @@ extern "C" void ag_rt_host_free(void *ptr, int pinned)
 /* ------------------------------------------------ device-to-host copies */
 #define AG_STAGE_CHUNK ((size_t)4 << 20)
 
+/* Page-locked staging of device-to-host copies: two chunks, and room for a
+ * solve's control record.  One copy uses it at a time; a caller that finds it
+ * taken copies directly. */
 static struct
 {
-    unsigned char *buf; /* two page-locked chunks */
+    unsigned char *buf;
+    AgControl *ctl;
     cudaEvent_t ev[2];
-    int state;          /* 0: not set up, 1: ready, -1: unavailable */
-} g_stage = {nullptr, {nullptr, nullptr}, 0};
+    int state; /* 0: not set up, 1: ready, -1: unavailable */
+} g_stage = {nullptr, nullptr, {nullptr, nullptr}, 0};
+static std::mutex g_stage_lock;
+
+/* the staging is set up and this thread's until `hold` goes */
+static bool stage_take(std::unique_lock<std::mutex> &hold)
+{
+    hold = std::unique_lock<std::mutex>(g_stage_lock, std::try_to_lock);
+    if (!hold.owns_lock())
+        return false;
+    if (g_stage.state == 0) {
+        g_stage.state = -1;
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, 2 * AG_STAGE_CHUNK + sizeof(AgControl), cudaHostAllocDefault) == cudaSuccess) {
+            if (cudaEventCreateWithFlags(&g_stage.ev[0], cudaEventDisableTiming) == cudaSuccess &&
+                cudaEventCreateWithFlags(&g_stage.ev[1], cudaEventDisableTiming) == cudaSuccess) {
+                g_stage.buf = (unsigned char *)p;
+                g_stage.ctl = (AgControl *)(g_stage.buf + 2 * AG_STAGE_CHUNK);
+                g_stage.state = 1;
+            } else {
+                cudaFreeHost(p);
+            }
+        }
+        cudaGetLastError();
+    }
+    if (g_stage.state != 1)
+        hold.unlock();
+    return g_stage.state == 1;
+}
 
 static ag_status_t event_wait(cudaEvent_t ev, double timeout_s)
 {
-    const double limit = wait_limit_s(timeout_s);
-    const double t0 = ag_wall_seconds();
-    unsigned spins = 0;
-    for (;;) {
-        cudaError_t e = cudaEventQuery(ev);
-        if (e == cudaSuccess)
-            return AG_OK;
-        if (e != cudaErrorNotReady)
-            return ag_set_error(AG_ERR_CUDA, "device copy failed: %s", cudaGetErrorString(e));
-        if (ag_wall_seconds() - t0 > limit)
-            return ag_set_error(AG_ERR_TIMEOUT, "device copy did not finish within %.1f s", limit);
-        if (++spins > 64) {
-            struct timespec ts = {0, 5000};
-            nanosleep(&ts, nullptr);
-        }
-    }
+    return poll_wait([ev] { return cudaEventQuery(ev); }, "device work", timeout_s);
 }
 
 /* host memcpy split over up to 16 OpenMP threads (one thread copies about
@@ -252,11 +277,13 @@ static void par_memcpy(void *dst, const void *src, size_t n)
     }
 }
 
-/* Copy `bytes` of device memory to host memory `dst` on the library stream
- * and wait for it (bounded).  A page-locked destination is copied directly;
- * a pageable one goes through two page-locked chunks, so that the device
- * copy of one chunk overlaps the host copy of the other. */
-static ag_status_t copy_to_host(void *dst, const void *src, size_t bytes)
+/* Copy `bytes` of device memory to host memory `dst` behind the library
+ * stream's work and wait for it (bounded).  A page-locked destination is
+ * copied directly; a pageable one goes through two page-locked chunks
+ * (`staged`: the caller holds them), so that the device copy of one chunk
+ * overlaps the host copy of the other, and nothing is waited for before the
+ * first chunk is queued. */
+static ag_status_t copy_to_host(void *dst, const void *src, size_t bytes, bool staged = false)
 {
     cudaStream_t s = g_ctx.stream;
     if (!bytes)
@@ -267,21 +294,8 @@ static ag_status_t copy_to_host(void *dst, const void *src, size_t bytes)
         pinned = at.type == cudaMemoryTypeHost;
     else
         cudaGetLastError();
-    if (!pinned && bytes >= ((size_t)1 << 20) && g_stage.state == 0) {
-        g_stage.state = -1;
-        void *p = nullptr;
-        if (cudaHostAlloc(&p, 2 * AG_STAGE_CHUNK, cudaHostAllocDefault) == cudaSuccess) {
-            if (cudaEventCreateWithFlags(&g_stage.ev[0], cudaEventDisableTiming) == cudaSuccess &&
-                cudaEventCreateWithFlags(&g_stage.ev[1], cudaEventDisableTiming) == cudaSuccess) {
-                g_stage.buf = (unsigned char *)p;
-                g_stage.state = 1;
-            } else {
-                cudaFreeHost(p);
-            }
-        }
-        cudaGetLastError();
-    }
-    if (pinned || bytes < ((size_t)1 << 20) || g_stage.state != 1) {
+    std::unique_lock<std::mutex> hold;
+    if (pinned || !(staged || stage_take(hold))) {
         AG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
         return stream_wait(s, 0);
     }
@@ -306,6 +320,8 @@ static ag_status_t copy_to_host(void *dst, const void *src, size_t bytes)
     }
     return AG_OK;
 }
+
+extern "C" int32_t ag_rt_copy_to_host(void *dst, const void *src, size_t bytes) { return copy_to_host(dst, src, bytes); }
 
 /* ------------------------------------------------------- graph handle */
 /* the integer pulls, AG_PREC_FIXED64 .. AG_PREC_QUANT8: contribution width in
@@ -344,6 +360,7 @@ struct ag_graph_s
     uint32_t *perm, *inv;   /* relabelling (NULL with AG_UPLOAD_KEEP_ORDER)  */
     float *out;             /* normalised ranks, caller order                */
     float *xbuf, *ybuf;     /* SpMV vectors in device order                  */
+    float *hx, *hy;         /* a host SpMV's vectors, caller order           */
     uint32_t hot_n;         /* entries of the shared-memory hot table        */
     uint32_t warm_n;        /* ids below this may allocate L1 lines          */
     ag_tile_config tiles;   /* work-list and cache shape in use              */
@@ -490,6 +507,8 @@ extern "C" ag_status_t ag_graph_release(ag_graph_t g)
     dev_free(g->g_f64);
     delete g->gstart_host;
     dev_free(g->out);
+    dev_free(g->hx);
+    dev_free(g->hy);
     dev_free(g->xbuf);
     dev_free(g->ybuf);
     dev_free(g->outdeg);
@@ -1960,32 +1979,37 @@ extern "C" ag_status_t ag_pagerank_fetch(ag_graph_t g, float *ranks, ag_pr_resul
     if (!g->launched)
         return ag_set_error(AG_ERR_INVALID_ARG, "ag_pagerank_fetch: nothing launched on this graph");
     cudaStream_t s = g_ctx.stream;
-    ag_status_t st = stream_wait(s, 0);
+    ag_status_t st = AG_OK;
+    /* The record and the ranks are queued behind the solve and waited for
+     * once: the record's head, and of its history what the caller asked for
+     * (all of it is 80 KB, read back pageable it took 25 us). */
+    std::unique_lock<std::mutex> hold;
+    std::vector<AgControl> own;
+    const bool staged = stage_take(hold);
+    AgControl *hc = g_stage.ctl;
+    if (!staged) {
+        own.resize(1);
+        hc = own.data();
+    }
+    const bool history = hist_active || hist_error || hist_seconds;
+    const size_t nh = history ? std::min<size_t>(history_len, AG_MAX_HISTORY) : 0;
+    AG_CUDA(cudaMemcpyAsync(hc, g->ctl, offsetof(AgControl, hist_active), cudaMemcpyDeviceToHost, s));
+    if (nh) {
+        AG_CUDA(cudaMemcpyAsync(hc->hist_active, g->ctl->hist_active, nh * 4, cudaMemcpyDeviceToHost, s));
+        AG_CUDA(cudaMemcpyAsync(hc->hist_err, g->ctl->hist_err, nh * 8, cudaMemcpyDeviceToHost, s));
+        AG_CUDA(cudaMemcpyAsync(hc->hist_t, g->ctl->hist_t, nh * 8, cudaMemcpyDeviceToHost, s));
+    }
+    st = ranks && g->N ? copy_to_host(ranks, g->out, (size_t)g->N * 4, staged) : stream_wait(s, 0);
     if (st != AG_OK)
         return st;
-    AgControl *hc = (AgControl *)malloc(sizeof(AgControl));
-    if (!hc)
-        return ag_set_error(AG_ERR_OOM, "host allocation failed");
-    cudaError_t e = cudaMemcpy(hc, g->ctl, sizeof(AgControl), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) {
-        free(hc);
-        return ag_set_error(AG_ERR_CUDA, "control readback failed: %s", cudaGetErrorString(e));
-    }
-    if (ranks && g->N) {
-        st = copy_to_host(ranks, g->out, (size_t)g->N * 4);
-        if (st != AG_OK) {
-            free(hc);
-            return st;
-        }
-    }
     const uint32_t passes = hc->iter;
     if (res) {
         memset(res, 0, sizeof(*res));
         res->passes = passes;
         res->converged = hc->converged;
         res->iterations = hc->converged ? (passes ? passes - 1 : 0) : passes;
-        res->active_last = passes ? hc->hist_active[std::min<uint32_t>(passes, AG_MAX_HISTORY) - 1] : 0;
-        res->error_total = passes ? hc->hist_err[std::min<uint32_t>(passes, AG_MAX_HISTORY) - 1] : 0.0;
+        res->active_last = passes ? hc->last_active : 0;
+        res->error_total = passes ? hc->last_err : 0.0;
         res->rank_sum = hc->rank_sum;
         res->switch_pass = hc->switch_pass;
         float ms = 0.0f;
@@ -2004,7 +2028,6 @@ extern "C" ag_status_t ag_pagerank_fetch(ag_graph_t g, float *ranks, ag_pr_resul
         }
     }
     const uint32_t fault = hc->fault;
-    free(hc);
     if (fault & 2u) {
         /* the solve gave up part way: the next one starts with a fresh barrier */
         AG_CUDA(cudaMemset(g->sync, 0, AG_SYNC_WORDS * 4));
@@ -2068,18 +2091,22 @@ extern "C" ag_status_t ag_spmv_pull(ag_graph_t g, const float *x, float *y, uint
     if (g->N == 0)
         return AG_OK;
     ag_status_t st = AG_OK;
-    float *dx = nullptr, *dy = nullptr;
     cudaStream_t s = g_ctx.stream;
-    AG_CUDA(cudaMallocAsync((void **)&dx, (size_t)g->N * 4, s));
-    AG_CUDA(cudaMallocAsync((void **)&dy, (size_t)g->N * 4, s));
-    AG_CUDA(cudaMemcpyAsync(dx, x, (size_t)g->N * 4, cudaMemcpyHostToDevice, s));
-    st = ag_spmv_pull_device(g, dx, dy, mode);
-    if (st == AG_OK)
-        st = copy_to_host(y, dy, (size_t)g->N * 4);
-    cudaFreeAsync(dx, s);
-    cudaFreeAsync(dy, s);
-    ag_status_t w = stream_wait(s, 0);
-    return st != AG_OK ? st : w;
+    /* the vectors' device copies are kept with the handle */
+    if (!g->hx) {
+        float *hx = (float *)dev_alloc(g, (size_t)g->N * 4 + 16, &st);
+        float *hy = (float *)dev_alloc(g, (size_t)g->N * 4 + 16, &st);
+        if (st != AG_OK) {
+            dev_free(hx);
+            dev_free(hy);
+            return st;
+        }
+        g->hx = hx;
+        g->hy = hy;
+    }
+    AG_CUDA(cudaMemcpyAsync(g->hx, x, (size_t)g->N * 4, cudaMemcpyHostToDevice, s));
+    st = ag_spmv_pull_device(g, g->hx, g->hy, mode);
+    return st == AG_OK ? copy_to_host(y, g->hy, (size_t)g->N * 4) : st;
 }
 
 /* -------------------------------------------------------- FP64 oracle */
@@ -2267,8 +2294,11 @@ extern "C" ag_status_t ag_multigraph_fetch(ag_graph_t g, float *ranks, uint32_t 
     const uint32_t n = g->ngraphs;
     std::vector<uint32_t> h(4 * (size_t)n);
     std::vector<double> hd(2 * (size_t)n);
-    AG_CUDA(cudaMemcpy(h.data(), g->g_u32, h.size() * 4, cudaMemcpyDeviceToHost));
-    AG_CUDA(cudaMemcpy(hd.data(), g->g_f64, hd.size() * 8, cudaMemcpyDeviceToHost));
+    st = copy_to_host(h.data(), g->g_u32, h.size() * 4);
+    if (st == AG_OK)
+        st = copy_to_host(hd.data(), g->g_f64, hd.size() * 8);
+    if (st != AG_OK)
+        return st;
     for (uint32_t i = 0; i < n; ++i) {
         const uint32_t np = h[2 * (size_t)n + i], cv = h[3 * (size_t)n + i];
         if (passes)

@@ -1469,6 +1469,8 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         }
         c->prev_err = err;
         c->last_err_sum = sum;
+        c->last_err = err;
+        c->last_active = active;
         c->iter = P + 1;
         c->converged = conv ? 1u : 0u;
         const bool cont = !conv && (P + 1 < max_iter);
