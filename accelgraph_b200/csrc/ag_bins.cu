@@ -186,19 +186,21 @@ __global__ void ag_bins_hubs_kernel(const AgBinsArgs a)
     }
 }
 
-__global__ void __launch_bounds__(AG_BINS_BLK) ag_bins_ids_kernel(const uint32_t *off, const uint32_t *ids,
+/* T: ids or weights */
+template <typename T>
+__global__ void __launch_bounds__(AG_BINS_BLK) ag_bins_ids_kernel(const uint32_t *off, const T *ids,
                                                                   const AgBin *bins, const uint4 *hubs, uint32_t nhub,
                                                                   const uint32_t *brow, const uint32_t *ubase,
-                                                                  uint32_t *out)
+                                                                  T *out)
 {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (blockIdx.x < nhub) {
         const uint4 h = hubs[blockIdx.x];
         const uint32_t len = (h.w & (AG_BIN_HUB - 1u)) + 1u;
-        const uint32_t *src = ids + off[h.x] + (size_t)h.y * AG_BIN_HUB;
-        uint32_t *dst = out + (size_t)blockIdx.x * AG_BIN_HUB;
+        const T *src = ids + off[h.x] + (size_t)h.y * AG_BIN_HUB;
+        T *dst = out + (size_t)blockIdx.x * AG_BIN_HUB;
         for (uint32_t i = tid; i < AG_BIN_HUB; i += AG_BINS_BLK)
-            dst[i] = i < len ? src[i] : 0u;
+            dst[i] = i < len ? src[i] : T(0);
         return;
     }
     const uint32_t k = blockIdx.x - nhub;
@@ -208,19 +210,19 @@ __global__ void __launch_bounds__(AG_BINS_BLK) ag_bins_ids_kernel(const uint32_t
     for (uint32_t u = warp; u < units; u += AG_BINS_BLK / 32) {
         const uint32_t e = brow[lb + 32u * u + lane], len = e >> 16;
         const uint32_t o = len ? off[b.r0 + (e & 0xffffu)] : 0u;
-        uint32_t *dst = out + b.sbase + ubase[(lb >> 5) + u];
+        T *dst = out + b.sbase + ubase[(lb >> 5) + u];
         if (u < ulong) {
             for (int l = 0; l < 32; ++l) {
                 const uint32_t n = __shfl_sync(0xffffffffu, len, l), ob = __shfl_sync(0xffffffffu, o, l);
                 for (uint32_t i = lane; i < ((n + 3u) & ~3u); i += 32)
-                    dst[i] = i < n ? ids[ob + i] : 0u;
+                    dst[i] = i < n ? ids[ob + i] : T(0);
                 dst += (n + 3u) & ~3u;
             }
         } else {
             const uint32_t most = __shfl_sync(0xffffffffu, len, 0); /* longest first */
 #pragma unroll 4
             for (uint32_t i = 0; i < most; ++i)
-                dst[32u * i + lane] = i < len ? ids[o + i] : 0u;
+                dst[32u * i + lane] = i < len ? ids[o + i] : T(0);
         }
     }
 }
@@ -304,10 +306,14 @@ extern "C" cudaError_t ag_bins_rows(const uint32_t *row_off, uint32_t n, const u
     return cudaGetLastError();
 }
 
-extern "C" cudaError_t ag_bins_ids(const uint32_t *row_off, const uint32_t *ids, const AgBinPlan *b, cudaStream_t s)
+extern "C" cudaError_t ag_bins_ids(const uint32_t *row_off, const uint32_t *ids, const float *w, const AgBinPlan *b,
+                                   cudaStream_t s)
 {
-    if (b->nbins + b->nhub)
-        ag_bins_ids_kernel<<<b->nbins + b->nhub, AG_BINS_BLK, 0, s>>>(row_off, ids, b->bins, b->hubs, b->nhub, b->brow,
-                                                                     b->ubase, b->ids);
+    const uint32_t grid = b->nbins + b->nhub;
+    if (grid) {
+        ag_bins_ids_kernel<<<grid, AG_BINS_BLK, 0, s>>>(row_off, ids, b->bins, b->hubs, b->nhub, b->brow, b->ubase, b->ids);
+        if (b->w)
+            ag_bins_ids_kernel<<<grid, AG_BINS_BLK, 0, s>>>(row_off, w, b->bins, b->hubs, b->nhub, b->brow, b->ubase, b->w);
+    }
     return cudaGetLastError();
 }

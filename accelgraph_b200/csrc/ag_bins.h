@@ -58,6 +58,7 @@ typedef struct AgBinPlan
     uint4 *hubs;
     uint32_t *brow, *ubase;
     uint32_t *ids;             /* in slot order, hub chunks first              */
+    float *w;                  /* weights in the same order, or NULL           */
     uint64_t *pre;             /* planning: scanned weights (and hub chunks)   */
     void *tmp;
 } AgBinPlan;
@@ -73,8 +74,9 @@ void ag_bins_shape(AgBinPlan *b, uint64_t total, uint32_t quantum, uint32_t ngra
 /* bins, rows and hub chunks (the caller has allocated bins, hubs, brow, ubase) */
 cudaError_t ag_bins_rows(const uint32_t *row_off, uint32_t n, const uint32_t *gstart, uint32_t ngraphs, AgBinPlan *b,
                          cudaStream_t s);
-/* in-neighbour ids in slot order */
-cudaError_t ag_bins_ids(const uint32_t *row_off, const uint32_t *ids, const AgBinPlan *b, cudaStream_t s);
+/* in-neighbour ids (and weights) in slot order */
+cudaError_t ag_bins_ids(const uint32_t *row_off, const uint32_t *ids, const float *w, const AgBinPlan *b,
+                        cudaStream_t s);
 size_t ag_bins_brow_words(const AgBinPlan *b, uint32_t n);
 #ifdef __cplusplus
 }

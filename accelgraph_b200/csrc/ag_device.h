@@ -372,8 +372,6 @@ cudaError_t ag_relabel_by_out_degree(const uint32_t *off_old, const uint32_t *id
                                      const uint32_t *outdeg_old, uint32_t n, uint32_t e, uint32_t *perm,
                                      uint32_t *inv, uint32_t *off_new, uint32_t *ids_new, float *w_new,
                                      uint32_t *outdeg_new, cudaStream_t s);
-cudaError_t ag_permute_in(const uint32_t *perm, const float *x, float *x_new, uint32_t n, cudaStream_t s);
-cudaError_t ag_permute_out(const uint32_t *inv, const float *y_new, float *y, uint32_t n, cudaStream_t s);
 cudaError_t ag_pr_f64_run(const uint32_t *row_off, const uint32_t *ids, const uint32_t *outdeg, uint32_t N,
                           uint32_t max_iter, double tol, double *r, double *r2, double *c, double *maxdiff,
                           uint32_t *passes_out, cudaStream_t s);

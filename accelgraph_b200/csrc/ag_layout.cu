@@ -132,20 +132,6 @@ __global__ void ag_copy_rows_kernel(const uint32_t *perm, const uint32_t *inv, c
     }
 }
 
-/* x_new[i] = x[perm[i]] */
-__global__ void ag_permute_in_kernel(const uint32_t *perm, const float *x, float *x_new, uint32_t n)
-{
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        x_new[i] = x[perm[i]];
-}
-
-/* y[v] = y_new[inv[v]] */
-__global__ void ag_permute_out_kernel(const uint32_t *inv, const float *y_new, float *y, uint32_t n)
-{
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        y[v] = y_new[inv[v]];
-}
-
 static unsigned grid_for(uint64_t n, unsigned per_block)
 {
     uint64_t g = (n + per_block - 1) / per_block;
@@ -237,20 +223,4 @@ extern "C" cudaError_t ag_relabel_by_out_degree(const uint32_t *off_old, const u
     if (err != cudaSuccess)
         return err;
     return ag_relabel_rows(perm, inv, off_old, off_new, ids_old, ids_new, w_old, w_new, n, e, s);
-}
-
-extern "C" cudaError_t ag_permute_in(const uint32_t *perm, const float *x, float *x_new, uint32_t n, cudaStream_t s)
-{
-    if (n == 0)
-        return cudaSuccess;
-    ag_permute_in_kernel<<<grid_for(n, 256), 256, 0, s>>>(perm, x, x_new, n);
-    return cudaGetLastError();
-}
-
-extern "C" cudaError_t ag_permute_out(const uint32_t *inv, const float *y_new, float *y, uint32_t n, cudaStream_t s)
-{
-    if (n == 0)
-        return cudaSuccess;
-    ag_permute_out_kernel<<<grid_for(n, 256), 256, 0, s>>>(inv, y_new, y, n);
-    return cudaGetLastError();
 }

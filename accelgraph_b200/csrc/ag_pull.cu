@@ -1,7 +1,8 @@
 /*
- * ag_pull.cu -- sm_100a pass-by-pass kernels of the pull: the SpMV product, a
- * row partition's pass, and the passes of a large union of graphs.  Whole
- * solves run on the solve kernel (ag_solve.cu).
+ * ag_pull.cu -- sm_100a pass-by-pass kernels of the pull: a row partition's
+ * pass, the passes and products of a large union of graphs, and the products
+ * inside the push forms.  Whole solves, and products on whole graphs, run on
+ * the solve kernel (ag_solve.cu).
  *
  * One pull pass (reference: the host contribution loop pageRank.c:1026-1033,
  * the accelerator gather of the cu_PageRank CSR PULL compute units, whose arithmetic the RTL

@@ -359,7 +359,7 @@ struct ag_graph_s
     float *w;
     uint32_t *perm, *inv;   /* relabelling (NULL with AG_UPLOAD_KEEP_ORDER)  */
     float *out;             /* normalised ranks, caller order                */
-    float *xbuf, *ybuf;     /* SpMV vectors in device order                  */
+    float *xbuf;            /* SpMV input in device order                    */
     float *hx, *hy;         /* a host SpMV's vectors, caller order           */
     uint32_t hot_n;         /* entries of the shared-memory hot table        */
     uint32_t warm_n;        /* ids below this may allocate L1 lines          */
@@ -510,7 +510,6 @@ extern "C" ag_status_t ag_graph_release(ag_graph_t g)
     dev_free(g->hx);
     dev_free(g->hy);
     dev_free(g->xbuf);
-    dev_free(g->ybuf);
     dev_free(g->outdeg);
     dev_free(g->w);
     dev_free(g->tasks_fast);
@@ -530,6 +529,7 @@ extern "C" ag_status_t ag_graph_release(ag_graph_t g)
     dev_free(g->bin.brow);
     dev_free(g->bin.ubase);
     dev_free(g->bin.ids);
+    dev_free(g->bin.w);
     dev_free(g->bin.pre);
     dev_free(g->bin.tmp);
     dev_free(g->hub_sum);
@@ -543,6 +543,7 @@ extern "C" ag_status_t ag_graph_release(ag_graph_t g)
     dev_free(g->unit.hubs);
     dev_free(g->unit.hrow);
     dev_free(g->unit.ids);
+    dev_free(g->unit.w);
     dev_free(g->unit.cnt);
     dev_free(g->unit.tmp);
     dev_free(g->hub_tag);
@@ -697,6 +698,7 @@ static ag_status_t plan_bins(ag_graph_s *g, uint64_t total)
     b->brow = (uint32_t *)dev_alloc(g, words * 4, &st);
     b->ubase = (uint32_t *)dev_alloc(g, words / 32 * 4 + 16, &st);
     b->ids = (uint32_t *)dev_alloc(g, (size_t)b->nslots * 4, &st);
+    b->w = g->w ? (float *)dev_alloc(g, (size_t)b->nslots * 4, &st) : nullptr;
     g->hub_sum = (double *)dev_alloc(g, (size_t)b->nhub * 8, &st);
     g->hub_words = (uint4 *)dev_alloc(g, (size_t)b->nhub * AG_BIN_ROUNDS * 16, &st);
     g->hub_seen = (uint32_t *)dev_alloc(g, (size_t)b->nhub * 4, &st);
@@ -777,6 +779,7 @@ static ag_status_t plan_unit_ids(ag_graph_s *g, const uint32_t *totals)
     u->hubs = (uint4 *)dev_alloc(g, (size_t)u->nhub * sizeof(uint4), &st);
     u->hrow = (uint32_t *)dev_alloc(g, (size_t)u->nhrow * 4, &st);
     u->ids = (uint4 *)dev_alloc(g, ((size_t)u->nhub * (AG_BIN_HUB / 4) + u->quads) * 16, &st);
+    u->w = g->w ? (float4 *)dev_alloc(g, ((size_t)u->nhub * (AG_BIN_HUB / 4) + u->quads) * 16, &st) : nullptr;
     g->hub_sum = (double *)dev_alloc(g, (size_t)u->nhub * 8, &st);
     g->hub_words = (uint4 *)dev_alloc(g, (size_t)u->nhub * AG_BIN_ROUNDS * 16, &st);
     /* (a chunk reads up to two entries past its own) */
@@ -1114,15 +1117,21 @@ static ag_status_t upload_impl(const struct GraphCSR *graph, uint32_t flags, con
         w_old = nullptr;
     }
     if (units) {
-        UP(ag_units_ids(g->row_off, g->ids, N, &g->unit, s));
+        UP(ag_units_ids(g->row_off, g->ids, g->w, N, &g->unit, s));
         dev_free(g->unit.tmp);
         g->unit.tmp = nullptr;
     } else if (whole) {
-        UP(ag_bins_ids(g->row_off, g->ids, &g->bin, s));
+        UP(ag_bins_ids(g->row_off, g->ids, g->w, &g->bin, s));
         dev_free(g->bin.pre);
         dev_free(g->bin.tmp);
         g->bin.pre = nullptr;
         g->bin.tmp = nullptr;
+    }
+    if (whole && g->w) {
+        /* the products read them in plan order */
+        dev_free(g->w);
+        g->w = nullptr;
+        g->device_bytes -= (uint64_t)g->E4 * 4;
     }
     UP(cudaEventCreate(&g->ev0));
     UP(cudaEventCreate(&g->ev1));
@@ -1302,14 +1311,22 @@ static size_t loop_smem(const ag_graph_s *g, int prec)
  * round trip to L2: tens of seconds, far above the longest pass) */
 #define AG_GRID_SPINS (1u << 26)
 
-/* a solve, or parts of one, as cooperative launches of the solve kernel: one
- * CTA on every SM (fewer on a graph of fewer bins) */
-static ag_status_t solve_launch(ag_graph_s *g, int prec, int exact, int dd, const AgRunConfig &run)
+/* parameters and shape of a solve kernel launch on this graph: one CTA on
+ * every SM (fewer on a graph of fewer bins) */
+struct SolveShape
 {
-    cudaStream_t s = g_ctx.stream;
-    AgSolveParams q;
+    const void *kernel;
+    unsigned grid;
+    size_t smem;
+};
+
+static ag_status_t solve_shape(ag_graph_s *g, int mode, int prec, int exact, bool hot, AgSolveParams &q, SolveShape &sh)
+{
     memset(&q, 0, sizeof(q));
     q.p = base_params(g, exact);
+    if (!hot)
+        q.p.hot_n = 0;
+    q.w = g->bin.w;
     q.bins = g->bin.bins;
     q.hubs = g->bin.hubs;
     q.brow = g->bin.brow;
@@ -1349,6 +1366,7 @@ static ag_status_t solve_launch(ag_graph_s *g, int prec, int exact, int dd, cons
         q.ids = (const uint32_t *)u.ids;
         q.uids = u.ids + (size_t)u.nhub * (AG_BIN_HUB / 4);
         q.hub_tag = g->hub_tag;
+        q.w = (const float *)u.w;
         bufs = 0;
         work = q.nunits;
     }
@@ -1356,13 +1374,30 @@ static ag_status_t solve_launch(ag_graph_s *g, int prec, int exact, int dd, cons
     q.p.hot_n = std::min(q.p.hot_n, fit);
     q.p.hot_n16 = std::min<uint32_t>(2 * q.p.hot_n, g->N & ~63u);
     const size_t smem = (size_t)q.p.hot_n * 4 + bufs;
-    const void *k = ag_solve_kernel_ptr(dd ? AG_MODE_DD : g->ngraphs ? AG_MODE_MULTI : AG_MODE_PR, prec, exact,
-                                        q.nunits != 0);
+    const void *k = ag_solve_kernel_ptr(mode, prec, exact, q.nunits != 0);
     ag_status_t st = pull_kernel_prepare(k, smem);
     if (st != AG_OK)
         return st;
-    const unsigned grid = (unsigned)std::max<uint64_t>(
+    sh.kernel = k;
+    sh.smem = smem;
+    sh.grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((uint64_t)g_ctx.num_sms, work));
+    return AG_OK;
+}
+
+/* a solve, or parts of one, as cooperative launches of the solve kernel */
+static ag_status_t solve_launch(ag_graph_s *g, int prec, int exact, int dd, const AgRunConfig &run)
+{
+    cudaStream_t s = g_ctx.stream;
+    AgSolveParams q;
+    SolveShape sh;
+    ag_status_t st =
+        solve_shape(g, dd ? AG_MODE_DD : g->ngraphs ? AG_MODE_MULTI : AG_MODE_PR, prec, exact, true, q, sh);
+    if (st != AG_OK)
+        return st;
+    const void *k = sh.kernel;
+    const unsigned grid = sh.grid;
+    const size_t smem = sh.smem;
     AgRunConfig r = run;
     void *args[2] = {&q, &r};
     const char *mode = getenv("AG_LAUNCH_MODE");
@@ -2056,28 +2091,45 @@ extern "C" ag_status_t ag_spmv_pull_device(ag_graph_t g, const float *x, float *
     ag_status_t st = AG_OK;
     if (g->perm && !g->xbuf) {
         g->xbuf = (float *)dev_alloc(g, (size_t)g->N * 4 + 16, &st);
-        g->ybuf = (float *)dev_alloc(g, (size_t)g->N * 4 + 16, &st);
         if (st != AG_OK)
             return st;
     }
     const int exact = (mode & AG_SPMV_EXACT) ? 1 : 0;
-    AgPullParams p = base_params(g, exact);
-    /* caller order in and out; the product runs in device order */
-    if (g->perm)
-        AG_CUDA(ag_permute_in(g->perm, x, g->xbuf, g->N, s));
-    p.x = g->perm ? g->xbuf : x;
-    p.rank = g->perm ? g->ybuf : y;
+    const bool weighted = g->w || g->bin.w || g->unit.w;
+    const int wmode = (mode & AG_SPMV_UNIT) ? AG_SPMV_W_UNIT : weighted ? AG_SPMV_W_GRAPH : AG_SPMV_W_CONST;
+    const float *dx = g->perm ? g->xbuf : x; /* in device order */
     /* the hot table needs a 16-byte aligned vector */
-    if (((uintptr_t)p.x & 15u) != 0)
+    const bool hot = ((uintptr_t)dx & 15u) == 0;
+    if (g->sync) {
+        /* one launch: x into device order, the product, y in caller order */
+        AgSolveParams q;
+        SolveShape sh;
+        st = solve_shape(g, AG_MODE_SPMV, 0, exact, hot, q, sh);
+        if (st != AG_OK)
+            return st;
+        q.p.x = dx;
+        q.p.wmode = wmode;
+        q.x_in = g->perm ? x : nullptr;
+        q.x_dev = g->xbuf;
+        q.y = y;
+        AgRunConfig run;
+        memset(&run, 0, sizeof(run));
+        void *args[2] = {&q, &run};
+        AG_CUDA(cudaLaunchCooperativeKernel(sh.kernel, dim3(sh.grid), dim3(AG_SOLVE_BLK), args, sh.smem, s));
+        return AG_OK;
+    }
+    /* a large union: in caller order, no relabelling */
+    AgPullParams p = base_params(g, exact);
+    p.x = dx;
+    p.rank = y;
+    if (!hot)
         p.hot_n = 0;
-    p.wmode = (mode & AG_SPMV_UNIT) ? AG_SPMV_W_UNIT : (g->w ? AG_SPMV_W_GRAPH : AG_SPMV_W_CONST);
+    p.wmode = wmode;
     const void *k = ag_pull_kernel_ptr(AG_MODE_SPMV, exact);
     const size_t smem = (size_t)AG_STAGE_BYTES + (size_t)p.hot_n * 4;
     const unsigned grid = pull_grid(k, p.ntasks, smem);
     void *args[1] = {&p};
     AG_CUDA(cudaLaunchKernel(k, dim3(grid), dim3(AG_BLK), args, smem, s));
-    if (g->perm)
-        AG_CUDA(ag_permute_out(g->inv, g->ybuf, y, g->N, s));
     return AG_OK;
 }
 

@@ -39,6 +39,9 @@
  * row sums magnitudes and is on the worklist when the pass is the first or a
  * sign was set.
  * No result depends on which warp ran what.
+ * SpMV: one such pass over any vector.  The launch first puts x into device
+ * order (a grid barrier follows), reads the weights in the order of the ids,
+ * and writes y in caller order.
  *
  * What bounds a pass: on a small graph the chain of waits (barrier, bin, ids,
  * gathers, the longest row's adds, update), about 7 us at 1024 vertices, where
@@ -52,6 +55,13 @@
  * copy rate).  The pull kernel's EXACT order
  * adds a long row on one lane while the other 31 wait; here they add other
  * rows, and neighbouring rows' warps share L1 lines.
+ *
+ * SpMV, weighted, us per product, FAST and EXACT, as three launches (permute,
+ * product by rows of a task, permute) -> here: R-MAT 65 K vertices 33 -> 15.4
+ * and 66 -> 29; 1 M 93 -> 70 and 147 -> 97; 4 M 316 -> 222 and 443 -> 336;
+ * uniform degrees, 1.2 M 74 -> 70 and 82 -> 72; 4 M 207 -> 190 and 224 -> 190.
+ * The weights are 4 more streamed bytes per edge (8E + 20N bytes at the copy
+ * rate: 95 us at R-MAT 4 M); the gathers still bound it.
  */
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -348,6 +358,20 @@ __device__ __forceinline__ uint32_t ag_sv_low_exp(uint32_t pred, uint32_t next)
 
 #define AG_SV_NOT_KEPT 0xffffffffu
 
+/* one round of a hub row value by value (eight consecutive values per lane,
+ * lanes below `done` are in s), one lane after another */
+__device__ __forceinline__ float ag_sv_serial(const float *v, float s, uint32_t done)
+{
+#pragma unroll 4
+    for (; done < 32u; ++done) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            s = __fadd_rn(s, v[i]);
+        s = __shfl_sync(0xffffffffu, s, done);
+    }
+    return s;
+}
+
 /* ------------------------------------------------------------------ solve */
 template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
 {
@@ -426,11 +450,27 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         return ok;
     }
 
+    /* the end of a launch without a closing barrier: the last CTA to get here
+     * clears the counters */
+    __device__ __forceinline__ void leave()
+    {
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            if (atomicAdd(q.sync + AG_SYNC_COUNT, 1u) == gridDim.x - 1) {
+                q.sync[AG_SYNC_COUNT] = 0;
+                q.sync[AG_SYNC_BIN] = 0;
+                q.sync[AG_SYNC_KEPT] = 0;
+                __threadfence();
+            }
+        }
+    }
+
     /* ------------------------------------------------------------ gathers */
     __device__ __forceinline__ void start_pass()
     {
         const bool odd = (iter & 1u) != 0;
-        c_in32 = odd ? p.c32_1 : p.c32_0;
+        c_in32 = MODE == AG_MODE_SPMV ? p.x : odd ? p.c32_1 : p.c32_0;
         c_out32 = odd ? p.c32_0 : p.c32_1;
         c_in16 = odd ? p.c16_1 : p.c16_0;
         c_out16 = odd ? p.c16_0 : p.c16_1;
@@ -472,10 +512,27 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         return u < hot_n ? hot32[u] : ag_sv_ld_f32(c_in32 + u, pol_last, u < p.warm_n);
     }
 
-    /* the group gathers `n` slots (a multiple of 4 is staged) from `ids` */
-    __device__ __forceinline__ void stage(float *vals, const uint32_t *ids, uint32_t n) const
+    /* SpMV: the weights of a quad (quad k of q.ids) */
+    __device__ __forceinline__ float4 weights(size_t k) const
     {
-        const uint4 *i4 = reinterpret_cast<const uint4 *>(ids);
+        if (p.wmode == AG_SPMV_W_GRAPH)
+            return ag_ld_stream_f4(reinterpret_cast<const float4 *>(q.w) + k, pol_first);
+        return p.wmode == AG_SPMV_W_CONST ? make_float4(0.0001f, 0.0001f, 0.0001f, 0.0001f)
+                                          : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    }
+
+    __device__ __forceinline__ static void times(float4 &x, const float4 &w)
+    {
+        x.x = __fmul_rn(w.x, x.x);
+        x.y = __fmul_rn(w.y, x.y);
+        x.z = __fmul_rn(w.z, x.z);
+        x.w = __fmul_rn(w.w, x.w);
+    }
+
+    /* the group gathers `n` slots (a multiple of 4 is staged) from slot k0 */
+    __device__ __forceinline__ void stage(float *vals, uint64_t k0, uint32_t n) const
+    {
+        const uint4 *i4 = reinterpret_cast<const uint4 *>(q.ids + k0);
         const uint32_t n4 = (n + 3u) >> 2;
         for (uint32_t i = st; i < n4; i += 2u * AG_SUB_THREADS) {
             const bool two = i + AG_SUB_THREADS < n4;
@@ -492,6 +549,11 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             y.y = gather(b.y);
             y.z = gather(b.z);
             y.w = gather(b.w);
+            if (MODE == AG_MODE_SPMV) {
+                const float4 wx = weights((k0 >> 2) + i), wy = weights((k0 >> 2) + i + (two ? AG_SUB_THREADS : 0u));
+                times(x, wx);
+                times(y, wy);
+            }
             reinterpret_cast<float4 *>(vals)[i] = x;
             if (two)
                 reinterpret_cast<float4 *>(vals)[i + AG_SUB_THREADS] = y;
@@ -514,6 +576,11 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
      * (sign cleared, pageRank.c:2896-2916) */
     __device__ __forceinline__ void finish(uint32_t at, uint32_t r, float s, float rp, uint32_t od)
     {
+        if (MODE == AG_MODE_SPMV) {
+            /* a sum that starts at +0 never ends at -0 */
+            q.y[p.perm ? __ldg(p.perm + r) : r] = __fadd_rn(s, 0.0f);
+            return;
+        }
         if (MODE == AG_MODE_DD) {
             if (iter == 0 || (__float_as_uint(s) >> 31)) {
                 const float rn = __fadd_rn(p.base, __fmul_rn(p.damp, fabsf(s)));
@@ -556,7 +623,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         const uint32_t nslots = hb.x, gid = hb.y;
         if (MODE == AG_MODE_MULTI && (nrows == 0 || *((volatile uint32_t *)(p.g_done + gid))))
             return; /* the same for the whole group */
-        const uint32_t *ids = q.ids + ((uint64_t)hb.z | ((uint64_t)hb.w << 32));
+        const uint64_t k0 = (uint64_t)hb.z | ((uint64_t)hb.w << 32);
         const uint32_t lb = ag_bin_list(r0, k);
         float *sums = vals + ((nslots + 3u) & ~3u);
         /* what the sums and the update need first is on its way while the
@@ -567,11 +634,11 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             e = __ldg(q.brow + lb + 32u * sw + lane);
             ub = __ldg(q.ubase + (lb >> 5) + sw);
         }
-        if (st < nrows) {
+        if (MODE != AG_MODE_SPMV && st < nrows) {
             rp = ag_ld_rank(p.rank + r0 + st);
             od = ag_ld_row_u32(p.outdeg + r0 + st);
         }
-        stage(vals, ids, nslots);
+        stage(vals, k0, nslots);
         /* rows without in-edges sum to 0; a hub row is its composer's */
         if (nrows > ha.z + ha.w)
             for (uint32_t i = st; i < nrows; i += AG_SUB_THREADS) {
@@ -639,7 +706,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         for (uint32_t i = st; i < nrows; i += AG_SUB_THREADS) {
             float rn = 0.0f;
             uint32_t on = 0;
-            if (i + AG_SUB_THREADS < nrows) {
+            if (MODE != AG_MODE_SPMV && i + AG_SUB_THREADS < nrows) {
                 rn = ag_ld_rank(p.rank + r0 + i + AG_SUB_THREADS);
                 on = ag_ld_row_u32(p.outdeg + r0 + i + AG_SUB_THREADS);
             }
@@ -728,7 +795,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         if (EXACT)
             for (uint32_t i = st; i <= nc * AG_BIN_ROUNDS; i += AG_SUB_THREADS)
                 sh.pred[sub][i] = __ldcg(q.hub_pred + (size_t)c0 * AG_BIN_ROUNDS + i);
-        stage(vals, q.ids + (size_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
+        stage(vals, (uint64_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
         ag_sv_sub_sync(sub);
         if (EXACT) {
             for (uint32_t t = sw; t < nc * AG_BIN_ROUNDS; t += AG_SUB_WARPS) {
@@ -804,7 +871,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                 q.hub_seen[h.z] = 0;
                 const uint32_t r = h.x;
                 if (MODE != AG_MODE_MULTI || !*((volatile uint32_t *)(p.g_done + graph_of(r))))
-                    finish(r, r, s, ag_ld_rank(p.rank + r), ag_ld_row_u32(p.outdeg + r));
+                    finish(r, r, s, MODE == AG_MODE_SPMV ? 0.0f : ag_ld_rank(p.rank + r), ag_ld_row_u32(p.outdeg + r));
             }
             __syncwarp();
             if (MODE == AG_MODE_MULTI)
@@ -825,7 +892,6 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         const size_t k0 = (size_t)h.z * AG_BIN_ROUNDS;
         const uint4 *words = q.hub_words + k0;
         uint16_t *pred = q.hub_pred + k0;
-        const uint4 *ids = reinterpret_cast<const uint4 *>(q.ids) + k0 * (AG_BIN_ROUND / 4);
         float s = (float)__ldcg(q.hub_sum + h.z);
         uint4 wn = make_uint4(0, 0, 0, 0);
         uint32_t en = 0, em = 0;
@@ -845,6 +911,10 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             }
             const bool live = k < rounds && k >= AG_BIN_HEAD / AG_BIN_ROUND;
             uint32_t done = b ? 0u : AG_BIN_HEAD / AG_BIN_ROUND;
+            /* rounds without a map at all */
+            uint32_t none = 0;
+            if (MODE == AG_MODE_SPMV)
+                none = __ballot_sync(0xffffffffu, live && (w.x & w.y & AG_XNOT) && w.z == AG_SV_NOT_KEPT);
             while (done < 32u && b + done < rounds) {
                 const uint32_t sb = __float_as_uint(s), ex = sb >> 23;
                 const uint32_t m = (sb & 0x7fffffu) | 0x800000u;
@@ -858,9 +928,13 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                         d1 = d0 + ((x >> 26) & 3u) - 1u;
                     }
                 }
-                ag_sv_scan(lane, d0, d1);
-                const uint32_t to = m + ((m & 1u) ? d1 : d0);
-                const uint32_t ok = __ballot_sync(0xffffffffu, to < (1u << 24));
+                uint32_t ok = ~(1u << done);
+                uint32_t to = 0;
+                if (MODE != AG_MODE_SPMV || !((none >> done) & 1u)) {
+                    ag_sv_scan(lane, d0, d1);
+                    to = m + ((m & 1u) ? d1 : d0);
+                    ok = __ballot_sync(0xffffffffu, to < (1u << 24));
+                }
                 const uint32_t out = ok == 0xffffffffu ? 32u : __ffs(~ok) - 1;
                 const uint32_t before = __shfl_sync(0xffffffffu, to, (out - 1u) & 31u);
                 const uint32_t prev = __shfl_up_sync(0xffffffffu, to, 1);
@@ -890,13 +964,34 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                             from = mapped(mp.z, mp.w, v, from, s);
                     }
                 } else {
-                    const uint4 x = __ldg(ids + (size_t)r * (AG_BIN_ROUND / 4) + 2 * lane);
-                    const uint4 y = __ldg(ids + (size_t)r * (AG_BIN_ROUND / 4) + 2 * lane + 1);
-                    gather8(x, y, r * AG_BIN_ROUND + 8u * lane, deg, v);
+                    const size_t kq = (k0 + r) * (AG_BIN_ROUND / 4) + 2u * lane;
+                    const uint4 *src = reinterpret_cast<const uint4 *>(q.ids) + kq;
+                    if (MODE == AG_MODE_SPMV && out < 31u && ((none >> out) & 2u)) {
+                        /* the next round is one of these too */
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(src + AG_BIN_ROUND / 4));
+                        if (p.wmode == AG_SPMV_W_GRAPH)
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float4 *>(q.w) + kq +
+                                                                         AG_BIN_ROUND / 4));
+                    }
+                    gather8(__ldg(src), __ldg(src + 1), r * AG_BIN_ROUND + 8u * lane, deg, kq, kq + 1, v);
                     if (MODE == AG_MODE_DD)
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
                             v[i] = fabsf(v[i]);
+                }
+                /* SpMV: a value below zero moves M back, so no map holds and the
+                 * round is added value by value.  EXACT, R-MAT of 1 M vertices,
+                 * x centred on 0: 447 us by the three launches, 418 here, the
+                 * largest row's chain; one x in 1000 below zero: 317 and 278 */
+                if (MODE == AG_MODE_SPMV) {
+                    bool bad = false;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        bad |= !(v[i] >= 0.0f);
+                    if (__any_sync(0xffffffffu, bad)) {
+                        s = ag_sv_serial(v, s, from);
+                        from = 32u;
+                    }
                 }
                 if (from < 32u)
                     s = ag_sv_round(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], s, lane, from);
@@ -941,7 +1036,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     {
         for (uint32_t k = blockIdx.x + sub * gridDim.x; k < q.nhb; k += gridDim.x * AG_SUBS) {
             const uint32_t c0 = k * q.per_bin, nc = min(q.per_bin, q.nhub - c0);
-            stage(vals, q.ids + (size_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
+            stage(vals, (uint64_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
             ag_sv_sub_sync(sub);
             for (uint32_t t = sw; t < nc * AG_BIN_ROUNDS; t += AG_SUB_WARPS) {
                 const uint4 h = __ldg(q.hubs + c0 + t / AG_BIN_ROUNDS);
@@ -997,18 +1092,32 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     }
 
     /* -------------------------------------------------------------- units */
-    /* eight gathered values of a lane's two quads; those at or past n are -0
-     * (s + -0 = s) */
-    __device__ __forceinline__ void gather8(const uint4 &a, const uint4 &b, uint32_t j, uint32_t n, float *v) const
+    /* eight gathered values of a lane's two quads (quads ka and kb of q.ids);
+     * those at or past n are -0 (s + -0 = s) */
+    __device__ __forceinline__ void gather8(const uint4 &a, const uint4 &b, uint32_t j, uint32_t n, size_t ka, size_t kb,
+                                            float *v) const
     {
-        v[0] = gather(a.x);
-        v[1] = gather(a.y);
-        v[2] = gather(a.z);
-        v[3] = gather(a.w);
-        v[4] = gather(b.x);
-        v[5] = gather(b.y);
-        v[6] = gather(b.z);
-        v[7] = gather(b.w);
+        float4 x, y, wx = make_float4(0.0f, 0.0f, 0.0f, 0.0f), wy = wx;
+        if (MODE == AG_MODE_SPMV) {
+            if (j < n)
+                wx = weights(ka);
+            if (j + 4u < n)
+                wy = weights(kb);
+        }
+        x.x = gather(a.x);
+        x.y = gather(a.y);
+        x.z = gather(a.z);
+        x.w = gather(a.w);
+        y.x = gather(b.x);
+        y.y = gather(b.y);
+        y.z = gather(b.z);
+        y.w = gather(b.w);
+        if (MODE == AG_MODE_SPMV) {
+            times(x, wx);
+            times(y, wy);
+        }
+        v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+        v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             if (j + i >= n)
@@ -1072,7 +1181,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             if (i + 2 < rounds)
                 pair(b0 + 32u * (i + 2), rounds - i - 2, na, nb);
             float v[8];
-            gather8(a, b, 4u * i, n, v);
+            gather8(a, b, 4u * i, n, unit_quad(b0, i), unit_quad(b0, i + 1), v);
             add8(sum, v, n);
             a = na;
             b = nb;
@@ -1147,7 +1256,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                     else
                         pair(bn, first_n, na, nb);
                     float v[8];
-                    gather8(a, b, 4u * i, n, v);
+                    gather8(a, b, 4u * i, n, unit_quad(b0, i), unit_quad(b0, i + 1), v);
                     add8(sum, v, n);
                     a = na;
                     b = nb;
@@ -1184,9 +1293,17 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         const uint32_t at = 32u * u + lane;
         if (at < p.N) {
             info = ag_ld_row_u32(q.info + at);
-            rp = ag_ld_rank(p.rank + at);
-            od = ag_ld_row_u32(q.uoutdeg + at);
+            if (MODE != AG_MODE_SPMV) {
+                rp = ag_ld_rank(p.rank + at);
+                od = ag_ld_row_u32(q.uoutdeg + at);
+            }
         }
+    }
+
+    /* quad i of this lane's row in a unit, as a quad of q.ids */
+    __device__ __forceinline__ size_t unit_quad(uint32_t b0, uint32_t i) const
+    {
+        return (size_t)q.nhub * (AG_BIN_HUB / 4) + b0 + 32u * i + lane;
     }
 
     /* this lane's quads at b0 and b0 + 32, as far as `left` rounds go */
@@ -1215,7 +1332,8 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                 nb = ag_ld_stream_u4(src + j / 4 + 3, pol_first);
             }
             float v[8];
-            gather8(a, b, j, AG_BIN_HEAD, v);
+            gather8(a, b, j, AG_BIN_HEAD, (size_t)first * (AG_BIN_HUB / 4) + j / 4,
+                    (size_t)first * (AG_BIN_HUB / 4) + j / 4 + 1, v);
             add8(sum, v, 0);
             a = na;
             b = nb;
@@ -1257,7 +1375,8 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                 nb = ag_ld_stream_u4(src + (rd + 1) * (AG_BIN_ROUND / 4) + 1, pol_first);
             }
             float v[8];
-            gather8(a, b, rd * AG_BIN_ROUND + 8u * lane, len, v);
+            const size_t kq = (size_t)c * (AG_BIN_HUB / 4) + rd * (AG_BIN_ROUND / 4) + 2u * lane;
+            gather8(a, b, rd * AG_BIN_ROUND + 8u * lane, len, kq, kq + 1, v);
             if (MODE == AG_MODE_DD) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -1313,7 +1432,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             const uint32_t at = __ldg(q.posof + h.x), nch = h.w >> 11;
             float rp = 0.0f;
             uint32_t od = 0, tag = 0;
-            if (lane == 0) {
+            if (MODE != AG_MODE_SPMV && lane == 0) {
                 rp = ag_ld_rank(p.rank + at);
                 od = ag_ld_row_u32(q.uoutdeg + at);
             }
@@ -1403,6 +1522,10 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             ag_sv_sub_sync(sub);
             k = sh.next[sub];
             ag_sv_sub_sync(sub);
+        }
+        if (MODE == AG_MODE_SPMV) {
+            leave();
+            return true;
         }
         /* CTA totals, then the last CTA closes the pass */
         {
@@ -1611,6 +1734,27 @@ __global__ void __launch_bounds__(AG_SOLVE_BLK, 1) ag_solve_kernel(const AgSolve
         ag_sv_mbar_init(&sh.mbar);
     s.gen = *((volatile uint32_t *)(q.sync + AG_SYNC_GEN));
     bool ok = true;
+    if (MODE == AG_MODE_SPMV) {
+        s.iter = 0;
+        s.eps = 0.0;
+        s.flags = 0;
+        __syncthreads();
+        if (q.x_in) {
+            const uint32_t n4 = q.p.N / 4u, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+            for (uint32_t v = t0; v < n4; v += gridDim.x * blockDim.x) {
+                const uint4 i = __ldg(reinterpret_cast<const uint4 *>(q.p.perm) + v);
+                const float4 x = make_float4(__ldg(q.x_in + i.x), __ldg(q.x_in + i.y), __ldg(q.x_in + i.z),
+                                             __ldg(q.x_in + i.w));
+                reinterpret_cast<float4 *>(q.x_dev)[v] = x;
+            }
+            if (t0 < (q.p.N & 3u))
+                q.x_dev[4u * n4 + t0] = __ldg(q.x_in + __ldg(q.p.perm + 4u * n4 + t0));
+            ok = s.grid_sync([&] { return 0u; });
+        }
+        if (ok)
+            s.pass(vals);
+        return;
+    }
     if (q.do_init) {
         s.init(run);
         const uint32_t f = (run.max_iter > 0 && q.p.N > 0 ? 0u : AG_GEN_STOP) |
@@ -1642,6 +1786,8 @@ extern "C" const void *ag_solve_kernel_ptr(int mode, int prec, int exact, int un
 {
     if (mode == AG_MODE_MULTI)
         return solve_ptr<AG_MODE_MULTI, 0, false>(exact);
+    if (mode == AG_MODE_SPMV)
+        return units ? solve_ptr<AG_MODE_SPMV, 0, true>(exact) : solve_ptr<AG_MODE_SPMV, 0, false>(exact);
     if (mode == AG_MODE_DD)
         return units ? solve_ptr<AG_MODE_DD, 0, true>(exact) : solve_ptr<AG_MODE_DD, 0, false>(exact);
     if (units)

@@ -31,6 +31,10 @@ typedef struct AgSolveParams
     const AgBin *bins;
     const uint4 *hubs;
     const uint32_t *brow, *ubase, *ids;
+    const float *w;           /* weights in the order of ids (SpMV)             */
+    const float *x_in;        /* SpMV: the vector in caller order, to be put in
+                                 device order in x_dev first (NULL: p.x is)     */
+    float *x_dev, *y;         /* SpMV: y in caller order                        */
     uint32_t nbins, nhub;     /* row bins, hub chunks                           */
     uint32_t per_bin, nhb;    /* hub chunks per bin, bins they make             */
     uint32_t buf;             /* floats of a group's buffer                     */

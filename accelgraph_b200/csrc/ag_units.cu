@@ -91,17 +91,19 @@ __global__ void ag_units_batches_kernel(AgUnitPlan u)
     }
 }
 
-__global__ void __launch_bounds__(256) ag_units_ids_kernel(const uint32_t *off, const uint32_t *ids, uint32_t n,
-                                                           const AgUnitPlan u)
+/* T, V: uint32_t, uint4 (ids) or float, float4 (weights) */
+template <typename T, typename V>
+__global__ void __launch_bounds__(256) ag_units_ids_kernel(const uint32_t *off, const T *ids, uint32_t n,
+                                                           const AgUnitPlan u, V *out)
 {
     const uint32_t tid = threadIdx.x, lane = tid & 31;
     if (blockIdx.x < u.nhub) {
         const uint4 h = u.hubs[blockIdx.x];
         const uint32_t len = (h.w & (AG_BIN_HUB - 1u)) + 1u;
-        const uint32_t *src = ids + off[h.x] + (size_t)h.y * AG_BIN_HUB;
-        uint32_t *dst = reinterpret_cast<uint32_t *>(u.ids) + (size_t)blockIdx.x * AG_BIN_HUB;
+        const T *src = ids + off[h.x] + (size_t)h.y * AG_BIN_HUB;
+        T *dst = reinterpret_cast<T *>(out) + (size_t)blockIdx.x * AG_BIN_HUB;
         for (uint32_t i = tid; i < AG_BIN_HUB; i += 256)
-            dst[i] = i < len ? src[i] : 0u;
+            dst[i] = i < len ? src[i] : T(0);
         return;
     }
     const uint32_t k = (blockIdx.x - u.nhub) * 8u + (tid >> 5);
@@ -109,15 +111,15 @@ __global__ void __launch_bounds__(256) ag_units_ids_kernel(const uint32_t *off, 
         return;
     const uint32_t at = 32u * k + lane;
     const uint32_t x = at < n ? u.info[at] : 0u, len = AG_UNIT_LEN(x);
-    const uint32_t *src = ids + (len ? off[(at & ~(AG_UNIT_WIN - 1u)) + AG_UNIT_ROW(x)] : 0u);
+    const T *src = ids + (len ? off[(at & ~(AG_UNIT_WIN - 1u)) + AG_UNIT_ROW(x)] : 0u);
     const uint32_t b0 = u.ubase[k], rounds = (u.ubase[k + 1] - b0) >> 5;
-    uint4 *dst = u.ids + (size_t)u.nhub * (AG_BIN_HUB / 4) + b0 + lane;
+    V *dst = out + (size_t)u.nhub * (AG_BIN_HUB / 4) + b0 + lane;
     for (uint32_t i = 0; i < rounds; ++i, dst += 32) {
-        uint4 q;
-        q.x = 4u * i < len ? src[4u * i] : 0u;
-        q.y = 4u * i + 1u < len ? src[4u * i + 1u] : 0u;
-        q.z = 4u * i + 2u < len ? src[4u * i + 2u] : 0u;
-        q.w = 4u * i + 3u < len ? src[4u * i + 3u] : 0u;
+        V q;
+        q.x = 4u * i < len ? src[4u * i] : T(0);
+        q.y = 4u * i + 1u < len ? src[4u * i + 1u] : T(0);
+        q.z = 4u * i + 2u < len ? src[4u * i + 2u] : T(0);
+        q.w = 4u * i + 3u < len ? src[4u * i + 3u] : T(0);
         *dst = q;
     }
 }
@@ -150,8 +152,8 @@ extern "C" uint32_t ag_units_batches(const AgUnitPlan *u, uint64_t quads)
     return (uint32_t)(w / u->batch) + 1u;
 }
 
-extern "C" cudaError_t ag_units_ids(const uint32_t *row_off, const uint32_t *ids, uint32_t n, const AgUnitPlan *u,
-                                    cudaStream_t s)
+extern "C" cudaError_t ag_units_ids(const uint32_t *row_off, const uint32_t *ids, const float *w, uint32_t n,
+                                    const AgUnitPlan *u, cudaStream_t s)
 {
     if (u->nhub) {
         cudaError_t e = cudaMemsetAsync(u->cnt, 0, 8, s);
@@ -161,7 +163,10 @@ extern "C" cudaError_t ag_units_ids(const uint32_t *row_off, const uint32_t *ids
     }
     ag_units_batches_kernel<<<ag_sm_grid(8), 256, 0, s>>>(*u);
     const uint32_t grid = u->nhub + (u->nunits + 7u) / 8u;
-    if (grid)
-        ag_units_ids_kernel<<<grid, 256, 0, s>>>(row_off, ids, n, *u);
+    if (grid) {
+        ag_units_ids_kernel<<<grid, 256, 0, s>>>(row_off, ids, n, *u, u->ids);
+        if (u->w)
+            ag_units_ids_kernel<<<grid, 256, 0, s>>>(row_off, w, n, *u, u->w);
+    }
     return cudaGetLastError();
 }

@@ -47,6 +47,7 @@ typedef struct AgUnitPlan
     uint4 *hubs;           /* hub chunks, as in ag_bins.h                     */
     uint32_t *hrow;        /* first chunk of each hub row                     */
     uint4 *ids;            /* hub chunks, then the units' quads               */
+    float4 *w;             /* weights in the same order, or NULL              */
     uint32_t *cnt;         /* planning: hub chunks, hub rows, heavy units     */
     void *tmp;
 } AgUnitPlan;
@@ -63,7 +64,8 @@ cudaError_t ag_units_rows(const uint32_t *row_off, const uint32_t *outdeg, uint3
 uint32_t ag_units_batches(const AgUnitPlan *u, uint64_t quads);
 /* hub chunks, batches and ids (the caller has allocated hubs, hrow, bstart,
  * ids and set nbatch) */
-cudaError_t ag_units_ids(const uint32_t *row_off, const uint32_t *ids, uint32_t n, const AgUnitPlan *u, cudaStream_t s);
+cudaError_t ag_units_ids(const uint32_t *row_off, const uint32_t *ids, const float *w, uint32_t n, const AgUnitPlan *u,
+                         cudaStream_t s);
 #ifdef __cplusplus
 }
 #endif
