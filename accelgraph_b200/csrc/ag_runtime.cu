@@ -2268,6 +2268,7 @@ extern "C" ag_status_t ag_rt_graph_view(ag_graph_t g, AgGraphView *v)
     v->tasks = g->tasks_fast;
     v->ntasks = g->ntasks_fast;
     v->hub_slots = g->nparts;
+    v->long_rows = g->bin.nhub || g->unit.nhub;
     return AG_OK;
 }
 

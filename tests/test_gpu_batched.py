@@ -72,3 +72,24 @@ def test_multigraph_iteration_cap_per_graph(gpu, oracle):
     for i, g in enumerate(gs):
         ref = oracle.pagerank_pull(g.in_edges_idx(), g.in_degree(), g.in_neighbours(), g.out_degree(), 7, 1e-9)
         assert info["iterations"][i] == ref["iterations"] and np.array_equal(parts[i], ref["ranks"])
+
+
+@pytest.mark.parametrize("k", [1, 7, 8, 9, 16, 17, 24, 31, 32, 33, 41, 63, 64])
+@pytest.mark.parametrize("longest", [1003, 2500])
+def test_ppr_column_widths(gpu, oracle, k, longest):
+    """Rows of 8, 16 and 32 lanes and row strides of every width class: each column bit for bit, with rows at the edges
+    of the shared-memory ring (more than 512 in-edges, groups of 8, ids by 32; at more than 32 columns
+    only with rows above 2048), empty rows and a ragged vertex count."""
+    ag = gpu
+    n = 1003
+    rng = np.random.default_rng(k)
+    lengths = [511, 512, 513, 519, 520, 521, 543, 544, 545, 639, 640, 641, longest, 0, 1]
+    src = np.concatenate([rng.integers(0, n, 9000)] + [rng.integers(0, n, m) for m in lengths]).astype(np.uint32)
+    dst = np.concatenate([rng.integers(20, n - 90, 9000), np.repeat(np.arange(len(lengths)), lengths)])
+    dst = dst.astype(np.uint32)
+    g = ag.Graph.from_edges(n, src, dst)
+    sources = rng.choice(n, k, replace=False).astype(np.uint32)
+    r, res = ag.DeviceGraph(g).ppr(sources, iterations=12, epsilon=1e-6)
+    ro, _, passes = oracle.ppr(g.in_edges_idx(), g.in_degree(), g.in_neighbours(), g.out_degree(), sources,
+                               iterations=12, epsilon=1e-6)
+    assert res.passes == passes and np.array_equal(r, ro)
