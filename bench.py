@@ -89,11 +89,11 @@ def dist_env():
 
 def profiled_traffic(scale: int, edge_factor: int, order: str):
     """DRAM bytes (read + write) of one pull pass of this kernel and graph from
-    the committed ncu summary profiles/ag_pull_kernel_<order>_rmat<scale>.md
+    the committed ncu summary profiles/ag_solve_kernel_<order>_rmat<scale>.md
     (row `dram__bytes_read.sum + write | R + W MB`), with the file it came
     from; (None, None) without one."""
     import re
-    name = f"profiles/ag_pull_kernel_{order}_rmat{scale}.md"
+    name = f"profiles/ag_solve_kernel_{order}_rmat{scale}.md"
     f = ROOT / name
     if edge_factor != 16 or not f.exists():
         return None, None
@@ -314,7 +314,7 @@ def run_b200(a):
     dev_pass = np.diff(np.concatenate([[0.0], np.cumsum(hist["seconds"])]))
     achieved = alg_bytes / pass_s / 1e9
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": None, "peak_kind": peak_kind, "kernel": "ag_pull_kernel<PR,fp32,%s>" % a.order,
+            "traffic": None, "peak_kind": peak_kind, "kernel": "ag_solve_kernel<PR,fp32,%s>" % a.order,
             "bytes_per_pass": alg_bytes, "pass_us": pass_s * 1e6,
             "pass_us_device_timer_median": float(np.median(dev_pass[1:]) * 1e6) if len(dev_pass) > 1 else None}
     if a.precision == 0:
@@ -369,7 +369,7 @@ def run_b200(a):
             "oracle": "C/OpenMP restatement of pageRankPullGraphCSR (pageRank.c:942-1109), same graph",
         }
 
-    launches = a.steps * (passes + 2)
+    launches = a.steps  # a solve is one launch of the solve kernel
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": a.steps, "warmup": a.warmup,
         "ms_per_step": t_max / a.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
