@@ -175,7 +175,9 @@ typedef struct ag_graph_info
     uint64_t device_bytes;   /* device memory held by the handle              */
 } ag_graph_info;
 
-/* Work-list and cache shape of a device graph (see ag_autotune). */
+/* Work-list and cache shape of a device graph (see ag_autotune).  Solves and
+ * products of whole graphs use hot_entries and warm_entries; the two first
+ * shape the work lists of the other forms. */
 typedef struct ag_tile_config
 {
     uint32_t task_edges;   /* in-edges per warp item of consecutive rows (32..256) */
@@ -201,7 +203,7 @@ ag_status_t ag_graph_release(ag_graph_t g);
 ag_status_t ag_graph_forget(const struct GraphCSR *graph);
 ag_status_t ag_graph_get_info(ag_graph_t g, ag_graph_info *info);
 ag_status_t ag_graph_get_tiles(ag_graph_t g, ag_tile_config *cfg);
-/* Copy a work list of the pull kernel (exact = 0: FAST order, 1: EXACT
+/* Copy a work list of the forms outside the solve kernel (exact = 0: FAST order, 1: EXACT
  * order) into `items` as 4 words per item (kind << 30 | first row, end row
  * or hub slot, first in-edge, end in-edge), in device row numbering;
  * *count receives the list's length.  At most `capacity` items are copied
@@ -209,7 +211,7 @@ ag_status_t ag_graph_get_tiles(ag_graph_t g, ag_tile_config *cfg);
 ag_status_t ag_graph_get_tasks(ag_graph_t g, int exact, uint32_t *items, uint32_t capacity, uint32_t *count);
 /* Re-plan the work list for another tile shape (results are unchanged in
  * EXACT order; FAST-order sums of rows split differently may differ in the
- * last bits). */
+ * last bits, in the forms that use the list). */
 ag_status_t ag_graph_set_tiles(ag_graph_t g, const ag_tile_config *cfg);
 /* Autotuner: time each candidate tile shape for `passes` pull passes on this
  * graph and keep the fastest; *best and *best_pass_us (may be NULL) receive
@@ -252,7 +254,7 @@ ag_status_t ag_autotune(ag_graph_t g, uint32_t passes, ag_tile_config *best, dou
 #define AG_DIR_PULL_PUSH 2
 
 #define AG_ORDER_FAST  0 /* rows of <= 32 in-edges summed in stream order,
-                            longer rows by a fixed lane-strided tree: ranks
+                            longer rows as trees of eight added in binary64: ranks
                             within 1e-5 relative L1 of the reference's, the
                             stopping pass not guaranteed equal               */
 #define AG_ORDER_EXACT 1 /* every row summed in stream order: bit-identical
@@ -329,8 +331,8 @@ ag_status_t ag_gather_uint(struct ag_graph_s *g, const void *x, uint32_t elem_by
 ag_status_t ag_pagerank_pull_ex(const struct Arguments *arguments, const struct GraphCSR *graph,
                                 const ag_pr_opts *opts, struct PageRankStats **out);
 
-/* Device-resident solve: enqueue init, the iteration loop (one CUDA graph with
- * an on-device convergence test) and normalisation on ag_stream().  Returns
+/* Device-resident solve: enqueue init, the iteration loop (with an on-device
+ * convergence test) and normalisation, as one launch, on ag_stream().  Returns
  * without waiting.  Results stay in the handle until the next launch. */
 ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations, double epsilon,
                                const ag_pr_opts *opts);
@@ -354,7 +356,7 @@ ag_status_t ag_pagerank_f64(ag_graph_t g, uint32_t max_iterations, double tol,
 /* --------------------------------------------- many independent graphs */
 /* Upload `count` graphs as one block-diagonal union (vertex ids of graph i
  * follow those of graph i-1).  ag_pagerank_launch on the handle then solves
- * every graph in the same CUDA-graph launch: one pass covers all graphs still
+ * every graph in the same launch: one pass covers all graphs still
  * running, each graph stops on its own convergence test or at the iteration
  * cap, and its items are skipped afterwards; ag_pagerank_fetch's ranks are
  * each graph's ranks normalised by its own vertex count, concatenated. */
