@@ -127,6 +127,19 @@ extern "C" int ag_num_sms(void)
 
 extern "C" const char *ag_version(void) { return "accelgraph-b200 0.1 sm_100a"; }
 
+/* a number from the environment, `otherwise` without a valid one */
+static uint32_t env_u32(const char *name, uint32_t otherwise)
+{
+    const char *env = getenv(name);
+    if (env && *env) {
+        char *end = nullptr;
+        const unsigned long v = strtoul(env, &end, 10);
+        if (end && *end == 0 && v <= 0xFFFFFFFFul)
+            return (uint32_t)v;
+    }
+    return otherwise;
+}
+
 static double wait_limit_s(double timeout_s)
 {
     if (timeout_s > 0)
@@ -323,6 +336,48 @@ static ag_status_t copy_to_host(void *dst, const void *src, size_t bytes, bool s
 
 extern "C" int32_t ag_rt_copy_to_host(void *dst, const void *src, size_t bytes) { return copy_to_host(dst, src, bytes); }
 
+/* --------------------------------------------- solve kernels that gave up */
+/* A solve kernel whose grid barrier ran out sets its graph's word in
+ * page-locked memory, so that a host call sees it without a copy of its own.
+ * The graph's device words stay marked, and its solves and products return at
+ * once, until solve_recover has cleared them.  Words are handed out in slabs
+ * that stay with the process and are used again. */
+#define AG_GAVE_UP_NEW 1u      /* set by the device: no call has reported it  */
+#define AG_GAVE_UP_REPORTED 2u /* reported; the words are not cleared yet     */
+#define AG_GAVE_UP_SLAB 1024u
+
+static std::mutex g_words_lock;
+static std::vector<volatile uint32_t *> g_words_slabs, g_words_free;
+
+static volatile uint32_t *word_take(void)
+{
+    std::lock_guard<std::mutex> hold(g_words_lock);
+    if (g_words_free.empty()) {
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, AG_GAVE_UP_SLAB * 4, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        g_words_slabs.push_back((volatile uint32_t *)p);
+        for (uint32_t i = AG_GAVE_UP_SLAB; i-- > 0;) {
+            ((volatile uint32_t *)p)[i] = 0;
+            g_words_free.push_back((volatile uint32_t *)p + i);
+        }
+    }
+    volatile uint32_t *w = g_words_free.back();
+    g_words_free.pop_back();
+    return w;
+}
+
+static void word_give(volatile uint32_t *w)
+{
+    if (!w)
+        return;
+    std::lock_guard<std::mutex> hold(g_words_lock);
+    *w = 0;
+    g_words_free.push_back(w);
+}
+
 /* ------------------------------------------------------- graph handle */
 /* the integer pulls, AG_PREC_FIXED64 .. AG_PREC_QUANT8: contribution width in
  * bytes and whether the form is quantised */
@@ -399,6 +454,8 @@ struct ag_graph_s
     float4 *hub_kept;
     uint32_t kept_cap;
     uint32_t *sync;
+    volatile uint32_t *gave_up; /* AG_GAVE_UP_*                              */
+    int on_solve;               /* the last launch was the solve kernel's    */
     /* the pull kernel's loop over a large union (FAST, EXACT) */
     AgExec exe[2];
     int have_exe[2];
@@ -560,6 +617,7 @@ extern "C" ag_status_t ag_graph_release(ag_graph_t g)
         cudaEventDestroy(g->ev1);
     if (g_ctx.ready)
         cudaStreamSynchronize(g_ctx.stream);
+    word_give(g->gave_up);
     delete g;
     return AG_OK;
 }
@@ -1081,6 +1139,8 @@ static ag_status_t upload_impl(const struct GraphCSR *graph, uint32_t flags, con
         st = plan_device(g, g->tiles.task_edges, g->tiles.hub_chunk);
     if (st == AG_OK && whole)
         st = units ? plan_unit_ids(g, unit_totals) : plan_bins(g, bin_total);
+    if (st == AG_OK && whole && !(g->gave_up = word_take()))
+        st = ag_set_error(AG_ERR_OOM, "page-locked allocation failed");
     if (st != AG_OK)
         UPFAIL(st);
 
@@ -1221,17 +1281,7 @@ static ag_status_t ensure_buffers(ag_graph_s *g, int prec)
 /* polls of the hot-table copy's mbarrier before a pull kernel reports the wait
  * as run out: AG_MBAR_SPINS (0 allowed: the first wait runs out at once, the
  * kernel flags it and then waits, bounded, for the copies) or 2^20 */
-static uint32_t mbar_spins(void)
-{
-    const char *env = getenv("AG_MBAR_SPINS");
-    if (env && *env) {
-        char *end = nullptr;
-        const unsigned long v = strtoul(env, &end, 10);
-        if (end && *end == 0 && v <= 0xFFFFFFFFul)
-            return (uint32_t)v;
-    }
-    return 1u << 20;
-}
+static uint32_t mbar_spins(void) { return env_u32("AG_MBAR_SPINS", 1u << 20); }
 
 static AgPullParams base_params(ag_graph_s *g, int exact)
 {
@@ -1307,9 +1357,47 @@ static size_t loop_smem(const ag_graph_s *g, int prec)
     return is_int_prec(prec) ? ag_fixed_smem_bytes(int_bytes(prec)) : pull_smem(g);
 }
 
-/* polls of a grid barrier of the solve kernel before it gives up (each a
- * round trip to L2: tens of seconds, far above the longest pass) */
-#define AG_GRID_SPINS (1u << 26)
+/* polls of a grid barrier of the solve kernel before it gives up:
+ * AG_GRID_SPINS (0 allowed: the first CTA to wait gives up at once) or 2^26
+ * (each a round trip to L2: tens of seconds, far above the longest pass) */
+static uint32_t grid_spins(void) { return env_u32("AG_GRID_SPINS", 1u << 26); }
+
+/* the graph's barrier and its hub rows' arrival counts as a new upload has
+ * them; runs behind whatever is queued */
+static ag_status_t solve_recover(ag_graph_s *g)
+{
+    AG_CUDA(cudaMemsetAsync(g->sync, 0, AG_SYNC_WORDS * 4, g_ctx.stream));
+    if (g->hub_seen && g->bin.nhub)
+        AG_CUDA(cudaMemsetAsync(g->hub_seen, 0, (size_t)g->bin.nhub * 4, g_ctx.stream));
+    *g->gave_up = 0;
+    return AG_OK;
+}
+
+/* Before a launch of the solve kernel: a barrier that ran out since the last
+ * one is reported by this call, unless it has been, and the graph is usable
+ * again. */
+static ag_status_t solve_ready(ag_graph_s *g)
+{
+    const uint32_t w = *g->gave_up;
+    if (w == 0)
+        return AG_OK;
+    ag_status_t st = solve_recover(g);
+    if (st == AG_OK && w == AG_GAVE_UP_NEW)
+        st = ag_set_error(AG_ERR_DEVICE_WAIT, "an earlier solve or product on this graph gave up at a grid barrier; "
+                          "it did not finish (nothing was launched now)");
+    return st;
+}
+
+/* After a wait for the solve kernel: whether it gave up */
+static ag_status_t solve_finished(ag_graph_s *g, const char *what)
+{
+    if (!g->gave_up || *g->gave_up == 0)
+        return AG_OK;
+    ag_status_t st = solve_recover(g);
+    return st != AG_OK ? st
+                       : ag_set_error(AG_ERR_DEVICE_WAIT, "a grid barrier of the solve kernel ran out before every CTA "
+                                      "arrived; the %s did not finish", what);
+}
 
 /* parameters and shape of a solve kernel launch on this graph: one CTA on
  * every SM (fewer on a graph of fewer bins) */
@@ -1344,7 +1432,8 @@ static ag_status_t solve_shape(ag_graph_s *g, int mode, int prec, int exact, boo
     q.kept_cap = g->kept_cap;
     q.hub_seen = g->hub_seen;
     q.sync = g->sync;
-    q.spins = AG_GRID_SPINS;
+    q.spins = grid_spins();
+    q.gave_up = g->gave_up;
     size_t bufs = (size_t)AG_SUBS * q.buf * 4;
     uint64_t work = (uint64_t)q.nhb + q.nbins;
     if (g->unit.nunits) {
@@ -1874,6 +1963,7 @@ static ag_status_t push_launch(ag_graph_s *g, const ag_pr_opts &o, uint32_t max_
     }
     AG_CUDA(cudaEventRecord(g->ev1, s));
     g->launched = 1;
+    g->on_solve = 0;
     g->last_prec = o.precision;
     g->last_exact = 0;
     return AG_OK;
@@ -1950,12 +2040,16 @@ extern "C" ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations,
     run.eps = epsilon;
     run.switch_residual = o.switch_residual > 0 ? o.switch_residual : 1e-4;
     if (!ip && g->sync) {
+        st = solve_ready(g);
+        if (st != AG_OK)
+            return st;
         AG_CUDA(cudaEventRecord(g->ev0, s));
         st = solve_launch(g, prec, exact, dd, run);
         if (st != AG_OK)
             return st;
         AG_CUDA(cudaEventRecord(g->ev1, s));
         g->launched = 1;
+        g->on_solve = 1;
         g->last_prec = prec;
         g->last_exact = exact;
         return AG_OK;
@@ -2001,6 +2095,7 @@ extern "C" ag_status_t ag_pagerank_launch(ag_graph_t g, uint32_t max_iterations,
     }
     AG_CUDA(cudaEventRecord(g->ev1, s));
     g->launched = 1;
+    g->on_solve = 0;
     g->last_prec = prec;
     g->last_exact = exact;
     return AG_OK;
@@ -2037,6 +2132,13 @@ extern "C" ag_status_t ag_pagerank_fetch(ag_graph_t g, float *ranks, ag_pr_resul
     st = ranks && g->N ? copy_to_host(ranks, g->out, (size_t)g->N * 4, staged) : stream_wait(s, 0);
     if (st != AG_OK)
         return st;
+    if (g->on_solve) {
+        st = solve_finished(g, "solve, or a product queued behind it,");
+        if (st != AG_OK) {
+            g->launched = 0; /* there is no result to fetch again */
+            return st;
+        }
+    }
     const uint32_t passes = hc->iter;
     if (res) {
         memset(res, 0, sizeof(*res));
@@ -2062,14 +2164,7 @@ extern "C" ag_status_t ag_pagerank_fetch(ag_graph_t g, float *ranks, ag_pr_resul
             hist_seconds[i] = (double)(hc->hist_t[i] - prev) * 1e-9;
         }
     }
-    const uint32_t fault = hc->fault;
-    if (fault & 2u) {
-        /* the solve gave up part way: the next one starts with a fresh barrier */
-        AG_CUDA(cudaMemset(g->sync, 0, AG_SYNC_WORDS * 4));
-        return ag_set_error(AG_ERR_DEVICE_WAIT, "a grid barrier of the solve kernel ran out before every CTA arrived; "
-                            "the solve did not finish");
-    }
-    if (fault)
+    if (hc->fault)
         return ag_set_error(AG_ERR_DEVICE_WAIT, "a pull kernel's bounded wait for its hot-table copy ran out "
                             "(the copies completed before the kernel went on; results are filled in)");
     return AG_OK;

@@ -372,6 +372,37 @@ __device__ __forceinline__ float ag_sv_serial(const float *v, float s, uint32_t 
     return s;
 }
 
+/* A CTA (one thread) waited in vain for barrier word `gen` to change; it found
+ * the arrival word at c when it arrived.  That word decides, once for all
+ * CTAs, how a barrier ends: it opens if all have arrived, else it is marked as
+ * given up, and whoever arrives later sees the mark.  Returns the barrier word
+ * as this CTA has to read it. */
+__device__ __noinline__ uint32_t ag_sv_give_up(uint32_t *sync, uint32_t gen, uint32_t c, uint32_t ctas,
+                                               volatile uint32_t *gave_up)
+{
+    uint32_t now = *((volatile uint32_t *)(sync + AG_SYNC_COUNT));
+    bool mine = false;
+    /* this barrier still, not given up, and not all there (at most one round
+     * for each CTA that arrives meanwhile) */
+    while (!mine && (c | now) < AG_COUNT_ABORT && ((now ^ c) & ~AG_COUNT_CTAS) == 0 && (now & AG_COUNT_CTAS) < ctas) {
+        const uint32_t was = atomicCAS(sync + AG_SYNC_COUNT, now, now | AG_COUNT_ABORT);
+        mine = was == now;
+        now = was;
+    }
+    uint32_t g = gen;
+    if (!mine && c < AG_COUNT_ABORT)
+        /* it opened, or another CTA gave it up: the word follows at once */
+        for (uint32_t i = 0; g == gen && i < 1u << 20; ++i)
+            asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(g) : "l"(sync + AG_SYNC_GEN) : "memory");
+    if (g == gen) {
+        g = gen | AG_GEN_ABORT;
+        atomicOr(sync + AG_SYNC_GEN, AG_GEN_ABORT);
+        *gave_up = 1u;
+        __threadfence_system();
+    }
+    return g;
+}
+
 /* ------------------------------------------------------------------ solve */
 template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
 {
@@ -412,22 +443,26 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     /* ------------------------------------------------------ grid barrier */
     /* every CTA's earlier writes are visible to every CTA after it; `close`
      * runs on the last CTA to arrive (all its threads) and returns the flags
-     * that the barrier hands on.  False (and ctl->fault) when the bounded wait
-     * ran out. */
+     * that the barrier hands on.  The wait is bounded: a CTA that waits in
+     * vain gives the barrier up for all (ag_sv_give_up), and then every CTA,
+     * late ones too, gets false here (or at the kernel's start) and runs
+     * nothing more. */
     template <typename F> __device__ __forceinline__ bool grid_sync(F close)
     {
+        uint32_t c = 0;
         __syncthreads();
         if (tid == 0) {
             __threadfence();
-            sh.last = atomicAdd(q.sync + AG_SYNC_COUNT, 1u) == gridDim.x - 1 ? 1u : 0u;
+            c = atomicAdd(q.sync + AG_SYNC_COUNT, 1u);
+            sh.last = (c & (AG_COUNT_ABORT | AG_COUNT_CTAS)) == gridDim.x - 1 ? 1u : 0u;
         }
         __syncthreads();
         if (sh.last) {
             __threadfence();
             const uint32_t f = close();
             if (tid == 0) {
-                const uint32_t g = (((gen >> 3) + 1u) << 3) | f;
-                q.sync[AG_SYNC_COUNT] = 0;
+                const uint32_t g = (((gen >> AG_GEN_SHIFT) + 1u) << AG_GEN_SHIFT) | f;
+                q.sync[AG_SYNC_COUNT] = ((c | AG_COUNT_CTAS) + 1u) & ~AG_COUNT_ABORT;
                 q.sync[AG_SYNC_BIN] = 0;
                 q.sync[AG_SYNC_KEPT] = 0;
                 sh.gen = g;
@@ -438,16 +473,15 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             uint32_t g = gen;
             for (uint32_t i = 0; g == gen && i < q.spins; ++i)
                 asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(g) : "l"(q.sync + AG_SYNC_GEN) : "memory");
+            if (g == gen)
+                g = ag_sv_give_up(q.sync, gen, c, gridDim.x, q.gave_up);
             sh.gen = g;
             __threadfence();
-            if (g == gen)
-                atomicOr(&p.ctl->fault, 2u);
         }
         __syncthreads();
-        const bool ok = sh.gen != gen;
         gen = sh.gen;
         flags = gen & 7u;
-        return ok;
+        return !(gen & AG_GEN_ABORT);
     }
 
     /* the end of a launch without a closing barrier: the last CTA to get here
@@ -457,8 +491,9 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         __syncthreads();
         if (tid == 0) {
             __threadfence();
-            if (atomicAdd(q.sync + AG_SYNC_COUNT, 1u) == gridDim.x - 1) {
-                q.sync[AG_SYNC_COUNT] = 0;
+            const uint32_t c = atomicAdd(q.sync + AG_SYNC_COUNT, 1u);
+            if ((c & AG_COUNT_CTAS) == gridDim.x - 1) {
+                q.sync[AG_SYNC_COUNT] = c & ~AG_COUNT_CTAS;
                 q.sync[AG_SYNC_BIN] = 0;
                 q.sync[AG_SYNC_KEPT] = 0;
                 __threadfence();
@@ -1730,15 +1765,20 @@ __global__ void __launch_bounds__(AG_SOLVE_BLK, 1) ag_solve_kernel(const AgSolve
     __shared__ AgSvShared sh;
     AgSolve<MODE, PREC, EXACT, UNITS> s(q, sh);
     float *vals = reinterpret_cast<float *>(ag_sv_dyn + (size_t)q.p.hot_n * 4) + (size_t)s.sub * q.buf;
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0) {
         ag_sv_mbar_init(&sh.mbar);
-    s.gen = *((volatile uint32_t *)(q.sync + AG_SYNC_GEN));
+        sh.gen = *((volatile uint32_t *)(q.sync + AG_SYNC_GEN));
+    }
+    /* one answer for the CTA: the word may change now if a barrier is given up */
+    __syncthreads();
+    s.gen = sh.gen;
+    if (s.gen & AG_GEN_ABORT)
+        return;
     bool ok = true;
     if (MODE == AG_MODE_SPMV) {
         s.iter = 0;
         s.eps = 0.0;
         s.flags = 0;
-        __syncthreads();
         if (q.x_in) {
             const uint32_t n4 = q.p.N / 4u, t0 = blockIdx.x * blockDim.x + threadIdx.x;
             for (uint32_t v = t0; v < n4; v += gridDim.x * blockDim.x) {

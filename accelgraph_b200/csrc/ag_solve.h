@@ -15,8 +15,9 @@
 #define AG_SUB_WARPS (AG_SUB_THREADS / 32)
 
 /* words of AgSolveParams::sync */
-#define AG_SYNC_COUNT 0       /* CTAs that have arrived                         */
-#define AG_SYNC_GEN 1         /* barriers passed << 3 | flags                   */
+#define AG_SYNC_COUNT 0       /* CTAs that have arrived at a barrier, how many
+                                 barriers were opened << 12, AG_COUNT_ABORT     */
+#define AG_SYNC_GEN 1         /* barriers passed << 4 | flags                   */
 #define AG_SYNC_BIN 2         /* bins handed out in this pass                   */
 #define AG_SYNC_KEPT 3        /* rounds kept in this pass                       */
 #define AG_SYNC_WORDS 4
@@ -24,6 +25,12 @@
 #define AG_GEN_STOP 1u
 #define AG_GEN_READ_LOW 2u
 #define AG_GEN_WRITE_LOW 4u
+#define AG_GEN_ABORT 8u       /* a CTA gave up waiting: no barrier of the graph
+                                 opens again until the host has cleared the
+                                 words                                          */
+#define AG_COUNT_ABORT 0x80000000u
+#define AG_COUNT_CTAS 0xfffu
+#define AG_GEN_SHIFT 4
 
 typedef struct AgSolveParams
 {
@@ -55,6 +62,8 @@ typedef struct AgSolveParams
     uint32_t *hub_tag;        /* units, data-driven: a sign was set; 2 x nhub    */
     uint32_t *sync;           /* AG_SYNC_WORDS                                  */
     uint32_t spins;           /* polls of a grid barrier before it gives up     */
+    volatile uint32_t *gave_up; /* page-locked word that the CTA which gives up
+                                 sets to 1                                      */
     uint32_t do_init, do_norm, max_pass; /* parts of a solve in this launch     */
 } AgSolveParams;
 

@@ -46,10 +46,13 @@ typedef int32_t ag_status_t;
 #define AG_ERR_TIMEOUT        -5  /* a bounded host wait ran out                  */
 #define AG_ERR_NO_DEVICE      -6  /* no usable CUDA device                        */
 #define AG_ERR_UNSUPPORTED    -7  /* option not available for this input          */
-#define AG_ERR_DEVICE_WAIT    -8  /* a bounded wait inside a kernel ran out (the
-                                     solve still finished; its results are
-                                     returned, but the device was not answering
-                                     in time)                                     */
+#define AG_ERR_DEVICE_WAIT    -8  /* a bounded wait inside a kernel ran out: for
+                                     the hot table's copy (the solve still
+                                     finished; its results are returned, but the
+                                     device was not answering in time), or at a
+                                     grid barrier (the solve or product did not
+                                     finish and has no results; the graph is
+                                     usable again).  ag_last_error() says which   */
 
 const char *ag_status_string(ag_status_t status);
 /* Detail of the most recent failure of this thread's last call ("" if none). */
