@@ -182,12 +182,16 @@ static ag_status_t stream_wait(cudaStream_t s, double timeout_s)
     return poll_wait([s] { return cudaStreamQuery(s); }, "device work", timeout_s);
 }
 
+static bool words_report(void);
+
 extern "C" ag_status_t ag_synchronize(double timeout_s)
 {
     ag_status_t st = ctx_ensure(-1);
-    if (st != AG_OK)
-        return st;
-    return stream_wait(g_ctx.stream, timeout_s);
+    if (st == AG_OK)
+        st = stream_wait(g_ctx.stream, timeout_s);
+    if (st == AG_OK && words_report())
+        st = ag_set_error(AG_ERR_DEVICE_WAIT, "a solve or product gave up at a grid barrier and did not finish");
+    return st;
 }
 
 extern "C" void *ag_rt_host_alloc(size_t bytes, int pinned, int *got_pinned)
@@ -367,6 +371,20 @@ static volatile uint32_t *word_take(void)
     volatile uint32_t *w = g_words_free.back();
     g_words_free.pop_back();
     return w;
+}
+
+/* whether a word was set that no call has reported yet */
+static bool words_report(void)
+{
+    std::lock_guard<std::mutex> hold(g_words_lock);
+    bool any = false;
+    for (volatile uint32_t *slab : g_words_slabs)
+        for (uint32_t i = 0; i < AG_GAVE_UP_SLAB; ++i)
+            if (slab[i] == AG_GAVE_UP_NEW) {
+                slab[i] = AG_GAVE_UP_REPORTED;
+                any = true;
+            }
+    return any;
 }
 
 static void word_give(volatile uint32_t *w)
@@ -2199,7 +2217,9 @@ extern "C" ag_status_t ag_spmv_pull_device(ag_graph_t g, const float *x, float *
         /* one launch: x into device order, the product, y in caller order */
         AgSolveParams q;
         SolveShape sh;
-        st = solve_shape(g, AG_MODE_SPMV, 0, exact, hot, q, sh);
+        st = solve_ready(g);
+        if (st == AG_OK)
+            st = solve_shape(g, AG_MODE_SPMV, 0, exact, hot, q, sh);
         if (st != AG_OK)
             return st;
         q.p.x = dx;
@@ -2253,7 +2273,9 @@ extern "C" ag_status_t ag_spmv_pull(ag_graph_t g, const float *x, float *y, uint
     }
     AG_CUDA(cudaMemcpyAsync(g->hx, x, (size_t)g->N * 4, cudaMemcpyHostToDevice, s));
     st = ag_spmv_pull_device(g, g->hx, g->hy, mode);
-    return st == AG_OK ? copy_to_host(y, g->hy, (size_t)g->N * 4) : st;
+    if (st == AG_OK)
+        st = copy_to_host(y, g->hy, (size_t)g->N * 4);
+    return st == AG_OK ? solve_finished(g, "product") : st;
 }
 
 /* -------------------------------------------------------- FP64 oracle */
@@ -2330,6 +2352,8 @@ extern "C" ag_status_t ag_spmv_run_host(ag_graph_t g, const float *x, float *y, 
             st = ag_set_error(AG_ERR_CUDA, "y readback failed: %s", cudaGetErrorString(e));
     }
     ag_status_t w = stream_wait(s, 0);
+    if (st == AG_OK && w == AG_OK)
+        st = solve_finished(g, "product");
     if (st == AG_OK && w == AG_OK && iter_seconds) {
         for (uint32_t i = 0; i < iterations; ++i) {
             float ms = 0.0f;

@@ -74,7 +74,9 @@ void *ag_stream(void);
 ag_status_t ag_set_stream(void *stream);
 /* Wait for the library stream, polling with a deadline (seconds; <=0 means
  * the AG_WAIT_TIMEOUT_S environment variable, default 600).  Returns
- * AG_ERR_TIMEOUT when the deadline passes with work still queued. */
+ * AG_ERR_TIMEOUT when the deadline passes with work still queued, and
+ * AG_ERR_DEVICE_WAIT when a solve or product that has ended gave up at a grid
+ * barrier and no other call has reported it. */
 ag_status_t ag_synchronize(double timeout_s);
 /* Number of streaming multiprocessors of the library's device (0 if none). */
 int ag_num_sms(void);
@@ -466,7 +468,9 @@ ag_status_t ag_mlp_warm_start_device(ag_graph_t g, ag_mlp_t m, float *init_ranks
                                     to a sequential binary32 loop)                */
 
 /* y = A x over the inverse CSR on ag_stream(); x and y are device pointers of
- * num_vertices floats.  Rows without in-edges get y[v] = 0. */
+ * num_vertices floats.  Rows without in-edges get y[v] = 0.  Returns without
+ * waiting: a product that gave up (AG_ERR_DEVICE_WAIT) is reported by
+ * ag_synchronize or by the next solve or product on the graph. */
 ag_status_t ag_spmv_pull_device(ag_graph_t g, const float *x, float *y, uint32_t mode);
 /* Host-pointer form: uploads x, runs, copies y back and waits. */
 ag_status_t ag_spmv_pull(ag_graph_t g, const float *x, float *y, uint32_t mode);

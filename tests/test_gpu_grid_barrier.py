@@ -57,3 +57,57 @@ def test_two_launches_before_a_fetch(gpu, oracle, monkeypatch):
     r, _, _ = dg.pagerank(6, 1e-6, order=ag.AG_ORDER_EXACT)
     assert np.array_equal(r, ref["ranks"])
     dg.release()
+
+
+@pytest.mark.parametrize("plan", ["bins", "units"])
+@pytest.mark.parametrize("exact", [0, 2])
+def test_product_gives_up_and_recovers(gpu, monkeypatch, plan, exact):
+    """A relabelled graph's product waits at a barrier: the host form reports it, the device form through
+    ag_synchronize or the graph's next call."""
+    import ctypes as C
+
+    import torch
+
+    ag = gpu
+    g = _graph(ag, _lengths(plan), 43)
+    n = g.num_vertices
+    dg = ag.DeviceGraph(g)
+    xh = np.random.default_rng(1).random(n, dtype=np.float32)
+    want = dg.spmv(xh, exact).view(np.uint32)
+    x, y = torch.from_numpy(xh).cuda(), torch.zeros(n, device="cuda")
+    torch.cuda.synchronize()
+
+    def product():
+        return ag.lib.ag_spmv_pull_device(dg.h, x.data_ptr(), y.data_ptr(), exact)
+
+    monkeypatch.setenv("AG_GRID_SPINS", "0")
+    with pytest.raises(ag.AGError) as err:
+        dg.spmv(xh, exact)
+    assert err.value.status == ag.AG_ERR_DEVICE_WAIT
+    assert product() == ag.AG_OK
+    assert ag.lib.ag_synchronize(C.c_double(60.0)) == ag.AG_ERR_DEVICE_WAIT
+    assert ag.lib.ag_synchronize(C.c_double(60.0)) == ag.AG_OK  # reported once
+    monkeypatch.delenv("AG_GRID_SPINS")
+    assert product() == ag.AG_OK and ag.lib.ag_synchronize(C.c_double(60.0)) == ag.AG_OK
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want)
+    monkeypatch.setenv("AG_GRID_SPINS", "0")
+    assert product() == ag.AG_OK
+    torch.cuda.synchronize()
+    monkeypatch.delenv("AG_GRID_SPINS")
+    assert product() == ag.AG_ERR_DEVICE_WAIT
+    assert np.array_equal(dg.spmv(xh, exact).view(np.uint32), want)
+    dg.release()
+
+
+def test_csr_product_reports(gpu, monkeypatch):
+    import ctypes as C
+
+    ag = gpu
+    g = _graph(ag, _lengths("bins"), 44)
+    args = ag.default_arguments(2, 1e-4)
+    out = C.POINTER(ag.SPMVStats)()
+    monkeypatch.setenv("AG_GRID_SPINS", "0")
+    assert ag.lib.ag_spmv_pull_ex(C.byref(args), g.ptr, 1, C.byref(out)) == ag.AG_ERR_DEVICE_WAIT
+    monkeypatch.delenv("AG_GRID_SPINS")
+    assert ag.lib.ag_spmv_pull_ex(C.byref(args), g.ptr, 1, C.byref(out)) == ag.AG_OK
+    ag.lib.freeSPMVStats(out)
