@@ -294,6 +294,15 @@ static void par_memcpy(void *dst, const void *src, size_t n)
     }
 }
 
+static bool page_locked(const void *p)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess)
+        return at.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return false;
+}
+
 /* Copy `bytes` of device memory to host memory `dst` behind the library
  * stream's work and wait for it (bounded).  A page-locked destination is
  * copied directly; a pageable one goes through two page-locked chunks
@@ -305,14 +314,8 @@ static ag_status_t copy_to_host(void *dst, const void *src, size_t bytes, bool s
     cudaStream_t s = g_ctx.stream;
     if (!bytes)
         return AG_OK;
-    cudaPointerAttributes at;
-    bool pinned = false;
-    if (cudaPointerGetAttributes(&at, dst) == cudaSuccess)
-        pinned = at.type == cudaMemoryTypeHost;
-    else
-        cudaGetLastError();
     std::unique_lock<std::mutex> hold;
-    if (pinned || !(staged || stage_take(hold))) {
+    if (page_locked(dst) || !(staged || stage_take(hold))) {
         AG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
         return stream_wait(s, 0);
     }
@@ -2147,7 +2150,14 @@ extern "C" ag_status_t ag_pagerank_fetch(ag_graph_t g, float *ranks, ag_pr_resul
         AG_CUDA(cudaMemcpyAsync(hc->hist_err, g->ctl->hist_err, nh * 8, cudaMemcpyDeviceToHost, s));
         AG_CUDA(cudaMemcpyAsync(hc->hist_t, g->ctl->hist_t, nh * 8, cudaMemcpyDeviceToHost, s));
     }
-    st = ranks && g->N ? copy_to_host(ranks, g->out, (size_t)g->N * 4, staged) : stream_wait(s, 0);
+    /* A page-locked `ranks` is lent for this call only: nothing is queued into
+     * it before the solve has ended, so that a wait that runs out leaves it
+     * alone. */
+    const bool want = ranks && g->N;
+    if (!want || page_locked(ranks))
+        st = stream_wait(s, 0);
+    if (st == AG_OK && want)
+        st = copy_to_host(ranks, g->out, (size_t)g->N * 4, staged);
     if (st != AG_OK)
         return st;
     if (g->on_solve) {

@@ -1,0 +1,35 @@
+"""What a fetch does to the caller's memory when its bounded wait runs out, and that it stays bounded."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+def test_timeout_leaves_the_buffer_alone(gpu, oracle, monkeypatch, pinned):
+    """ag_pagerank_fetch that timed out writes nothing into `ranks`, neither then nor when the solve ends; a second
+    fetch delivers."""
+    import torch
+
+    ag = gpu
+    g = ag.Graph.rmat(18, 16, seed=5)
+    ref = oracle.pagerank_pull(g.in_edges_idx(), g.in_degree(), g.in_neighbours(), g.out_degree(), 400, 0.0)
+    dg = ag.DeviceGraph(g)
+    dg.pagerank(2, 1e-6, order=ag.AG_ORDER_EXACT)
+    ranks = torch.full((g.num_vertices,), -7.0, pin_memory=pinned)
+    ptr, res = C.cast(ranks.data_ptr(), ag.f32p), ag.PRResult()
+
+    def fetch():
+        return ag.lib.ag_pagerank_fetch(dg.h, ptr, C.byref(res), None, None, None, 0)
+
+    dg.launch(400, 0.0, order=ag.AG_ORDER_EXACT)
+    monkeypatch.setenv("AG_WAIT_TIMEOUT_S", "1e-7")
+    assert fetch() == ag.AG_ERR_TIMEOUT
+    monkeypatch.delenv("AG_WAIT_TIMEOUT_S")
+    assert ag.lib.ag_synchronize(C.c_double(120.0)) == ag.AG_OK
+    assert (ranks.numpy() == -7.0).all()
+    assert fetch() == ag.AG_OK and res.passes == ref["passes"]
+    assert np.array_equal(ranks.numpy(), ref["ranks"])
+    dg.release()
