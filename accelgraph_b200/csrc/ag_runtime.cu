@@ -315,7 +315,12 @@ static ag_status_t copy_to_host(void *dst, const void *src, size_t bytes, bool s
     if (!bytes)
         return AG_OK;
     std::unique_lock<std::mutex> hold;
-    if (page_locked(dst) || !(staged || stage_take(hold))) {
+    const bool locked = page_locked(dst);
+    if (locked || !(staged || stage_take(hold))) {
+        /* the driver waits for a pageable copy, and without a limit */
+        ag_status_t st = locked ? AG_OK : stream_wait(s, 0);
+        if (st != AG_OK)
+            return st;
         AG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
         return stream_wait(s, 0);
     }
@@ -2141,6 +2146,10 @@ extern "C" ag_status_t ag_pagerank_fetch(ag_graph_t g, float *ranks, ag_pr_resul
     if (!staged) {
         own.resize(1);
         hc = own.data();
+        /* (the driver waits for a pageable copy, and without a limit) */
+        st = stream_wait(s, 0);
+        if (st != AG_OK)
+            return st;
     }
     const bool history = hist_active || hist_error || hist_seconds;
     const size_t nh = history ? std::min<size_t>(history_len, AG_MAX_HISTORY) : 0;

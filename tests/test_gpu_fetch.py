@@ -1,5 +1,7 @@
 """What a fetch does to the caller's memory when its bounded wait runs out, and that it stays bounded."""
 import ctypes as C
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -33,3 +35,29 @@ def test_timeout_leaves_the_buffer_alone(gpu, oracle, monkeypatch, pinned):
     assert fetch() == ag.AG_OK and res.passes == ref["passes"]
     assert np.array_equal(ranks.numpy(), ref["ranks"])
     dg.release()
+
+
+def test_fetch_beside_another_is_bounded(gpu, oracle, monkeypatch):
+    """While another thread's fetch holds the staging, a fetch copies directly; its wait for the solve still has the
+    limit that the caller set."""
+    ag = gpu
+    ga, gb = ag.Graph.rmat(20, 16, seed=6), ag.Graph.rmat(12, 16, seed=7)
+    ref = oracle.pagerank_pull(gb.in_edges_idx(), gb.in_degree(), gb.in_neighbours(), gb.out_degree(), 20, 1e-6)
+    da, db = ag.DeviceGraph(ga), ag.DeviceGraph(gb)
+    got = []
+    da.launch(4000, 0.0, order=ag.AG_ORDER_EXACT)  # some 0.3 s
+    thread = threading.Thread(target=lambda: got.append(da.fetch()[1].passes))
+    thread.start()
+    time.sleep(0.05)
+    db.launch(20, 1e-6, order=ag.AG_ORDER_EXACT)
+    monkeypatch.setenv("AG_WAIT_TIMEOUT_S", "1e-7")
+    with pytest.raises(ag.AGError) as err:
+        db.fetch()
+    assert err.value.status == ag.AG_ERR_TIMEOUT
+    monkeypatch.delenv("AG_WAIT_TIMEOUT_S")
+    thread.join()
+    assert got == [4000]
+    r, res, _ = db.fetch()
+    assert res.iterations == ref["iterations"] and np.array_equal(r, ref["ranks"])
+    da.release()
+    db.release()
