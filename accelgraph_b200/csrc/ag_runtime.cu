@@ -294,13 +294,13 @@ static void par_memcpy(void *dst, const void *src, size_t n)
     }
 }
 
-static bool page_locked(const void *p)
+static cudaMemoryType memory_type(const void *p)
 {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) == cudaSuccess)
-        return at.type == cudaMemoryTypeHost;
+        return at.type;
     cudaGetLastError();
-    return false;
+    return cudaMemoryTypeUnregistered;
 }
 
 /* Copy `bytes` of device memory to host memory `dst` behind the library
@@ -315,7 +315,10 @@ static ag_status_t copy_to_host(void *dst, const void *src, size_t bytes, bool s
     if (!bytes)
         return AG_OK;
     std::unique_lock<std::mutex> hold;
-    const bool locked = page_locked(dst);
+    const cudaMemoryType type = memory_type(dst);
+    const bool locked = type == cudaMemoryTypeHost;
+    if (type == cudaMemoryTypeDevice)
+        return ag_set_error(AG_ERR_INVALID_ARG, "a host destination is needed, not device memory");
     if (locked || !(staged || stage_take(hold))) {
         /* the driver waits for a pageable copy, and without a limit */
         ag_status_t st = locked ? AG_OK : stream_wait(s, 0);
@@ -2163,7 +2166,7 @@ extern "C" ag_status_t ag_pagerank_fetch(ag_graph_t g, float *ranks, ag_pr_resul
      * it before the solve has ended, so that a wait that runs out leaves it
      * alone. */
     const bool want = ranks && g->N;
-    if (!want || page_locked(ranks))
+    if (!want || memory_type(ranks) == cudaMemoryTypeHost)
         st = stream_wait(s, 0);
     if (st == AG_OK && want)
         st = copy_to_host(ranks, g->out, (size_t)g->N * 4, staged);

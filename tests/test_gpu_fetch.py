@@ -61,3 +61,22 @@ def test_fetch_beside_another_is_bounded(gpu, oracle, monkeypatch):
     assert res.iterations == ref["iterations"] and np.array_equal(r, ref["ranks"])
     da.release()
     db.release()
+
+
+def test_device_memory_as_the_host_destination_is_refused(gpu, oracle):
+    """The host reads and writes staged destinations itself: a device pointer is an error, not a crash."""
+    import torch
+
+    ag = gpu
+    g = ag.Graph.rmat(10, 8)
+    dg = ag.DeviceGraph(g)
+    buf = torch.zeros(g.num_vertices, device="cuda")
+    ptr = C.cast(buf.data_ptr(), ag.f32p)
+    dg.launch(5, 1e-6)
+    assert ag.lib.ag_pagerank_fetch(dg.h, ptr, None, None, None, None, 0) == ag.AG_ERR_INVALID_ARG
+    x = np.ones(g.num_vertices, np.float32)
+    assert ag.lib.ag_spmv_pull(dg.h, x.ctypes.data_as(ag.f32p), ptr, 0) == ag.AG_ERR_INVALID_ARG
+    assert ag.lib.ag_synchronize(C.c_double(60.0)) == ag.AG_OK and not buf.any()
+    want = oracle.spmv_pull(g.in_edges_idx(), g.in_degree(), g.in_neighbours(), np.ones(g.num_edges, np.float32), x)
+    assert np.array_equal(dg.spmv(x, ag.AG_SPMV_UNIT | ag.AG_SPMV_EXACT), want)
+    dg.release()
