@@ -2537,8 +2537,18 @@ extern "C" ag_status_t ag_graph_get_tasks(ag_graph_t g, int exact, uint32_t *ite
     return AG_OK;
 }
 
-/* re-plan the work lists for a new tile shape; cached launch graphs are
- * rebuilt on the next launch */
+/* sizes of the hot table and the warm tier; cached launch graphs are rebuilt
+ * on the next launch */
+static void set_tables(ag_graph_s *g, uint32_t hot, uint32_t warm)
+{
+    g->hot_n = g->hot_allowed ? std::min<uint32_t>(std::min<uint32_t>(hot, AG_HOT_MAX), g->N) & ~63u : 0u;
+    g->warm_n = std::max<uint32_t>(warm, g->hot_n);
+    g->tiles.hot_entries = g->hot_n;
+    g->tiles.warm_entries = g->warm_n;
+    drop_execs(g);
+}
+
+/* re-plan the work lists for a new tile shape */
 extern "C" ag_status_t ag_graph_set_tiles(ag_graph_t g, const ag_tile_config *cfg)
 {
     ag_clear_error();
@@ -2554,23 +2564,20 @@ extern "C" ag_status_t ag_graph_set_tiles(ag_graph_t g, const ag_tile_config *cf
     ag_status_t st = stream_wait(s, 0);
     if (st != AG_OK)
         return st;
-    const uint32_t N = g->N;
     st = plan_device(g, cfg->task_edges, cfg->hub_chunk);
     if (st != AG_OK)
         return st;
     g->tiles = *cfg;
-    g->hot_n = g->hot_allowed ? std::min<uint32_t>(std::min<uint32_t>(cfg->hot_entries, AG_HOT_MAX), N) & ~63u : 0u;
-    g->warm_n = std::max<uint32_t>(cfg->warm_entries, g->hot_n);
-    g->tiles.hot_entries = g->hot_n;
-    g->tiles.warm_entries = g->warm_n;
-    drop_execs(g);
+    set_tables(g, cfg->hot_entries, cfg->warm_entries);
     return stream_wait(s, 0);
 }
 
-/* Time each candidate tile shape on this graph (FP32, FAST order, a fixed
- * number of passes that never stop early) and keep the fastest.  Candidates:
- * item caps {128, 256}, hub chunks {1024, 2048, 4096}, and, when the
- * shared-memory table is allowed, table sizes {0, 8K, 16K, 24K} entries.
+/* Time each candidate tile shape on this graph (FP32, the default order, a
+ * fixed number of passes that never stop early) and keep the fastest.
+ * Candidates: table sizes {0, 8K, 16K, 24K} entries, when the shared-memory
+ * table is allowed; where solves run on the work list (unions above
+ * AG_UNION_MAX_EDGES), item caps {128, 256} and hub chunks {1024, 2048, 4096}.
+ * Elsewhere the timed solve does not read the list, which stays as it is.
  * With AG_TUNE_CACHE naming a file, results are read from and appended to it
  * (one line per graph shape: N E max-in-degree device cap chunk hot warm us). */
 extern "C" ag_status_t ag_autotune(ag_graph_t g, uint32_t passes, ag_tile_config *best, double *best_pass_us)
@@ -2592,6 +2599,15 @@ extern "C" ag_status_t ag_autotune(ag_graph_t g, uint32_t passes, ag_tile_config
                     *c = '_';
         }
     }
+    const bool on_list = !g->sync;
+    auto apply = [&](const ag_tile_config &c) -> ag_status_t {
+        if (on_list)
+            return ag_graph_set_tiles(g, &c);
+        ag_status_t st = stream_wait(g_ctx.stream, 0);
+        if (st == AG_OK)
+            set_tables(g, c.hot_entries, c.warm_entries);
+        return st;
+    };
     const char *cache = getenv("AG_TUNE_CACHE");
     if (cache) {
         FILE *f = fopen(cache, "r");
@@ -2603,7 +2619,7 @@ extern "C" ag_status_t ag_autotune(ag_graph_t g, uint32_t passes, ag_tile_config
                 if (n == g->N && e == g->E && md == g->max_in_degree && strcmp(dn, dev_name) == 0) {
                     ag_tile_config c = {cap, chunk, hot, warm};
                     fclose(f);
-                    ag_status_t st = ag_graph_set_tiles(g, &c);
+                    ag_status_t st = apply(c);
                     if (st == AG_OK) {
                         if (best)
                             *best = g->tiles;
@@ -2617,8 +2633,11 @@ extern "C" ag_status_t ag_autotune(ag_graph_t g, uint32_t passes, ag_tile_config
         }
     }
     std::vector<ag_tile_config> cands;
-    const uint32_t caps[2] = {128, 256};
-    const uint32_t chunks[3] = {1024, 2048, 4096};
+    std::vector<uint32_t> caps = {128, 256}, chunks = {1024, 2048, 4096};
+    if (!on_list) {
+        caps = {g->tiles.task_edges};
+        chunks = {g->tiles.hub_chunk};
+    }
     const uint32_t hots[4] = {0, 8192, 16384, 24576};
     const int nh = g->hot_allowed ? 4 : 1;
     for (uint32_t c : caps)
@@ -2631,7 +2650,7 @@ extern "C" ag_status_t ag_autotune(ag_graph_t g, uint32_t passes, ag_tile_config
     ag_pr_opts_init(&o);
     o.quiet = 1;
     for (const ag_tile_config &c : cands) {
-        ag_status_t st = ag_graph_set_tiles(g, &c);
+        ag_status_t st = apply(c);
         if (st != AG_OK)
             return st;
         ag_pr_result r;
@@ -2650,7 +2669,7 @@ extern "C" ag_status_t ag_autotune(ag_graph_t g, uint32_t passes, ag_tile_config
             bestc = g->tiles;
         }
     }
-    ag_status_t st = ag_graph_set_tiles(g, &bestc);
+    ag_status_t st = apply(bestc);
     if (st != AG_OK)
         return st;
     if (cache) {

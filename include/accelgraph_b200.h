@@ -220,7 +220,9 @@ ag_status_t ag_graph_get_tasks(ag_graph_t g, int exact, uint32_t *items, uint32_
 ag_status_t ag_graph_set_tiles(ag_graph_t g, const ag_tile_config *cfg);
 /* Autotuner: time each candidate tile shape for `passes` pull passes on this
  * graph and keep the fastest; *best and *best_pass_us (may be NULL) receive
- * it.  AG_TUNE_CACHE names an optional cache file of earlier results. */
+ * it.  Candidates differ in hot_entries and warm_entries; the work list, which
+ * the timed solve does not read, stays as it is (on a union whose solves do
+ * run on it, above 64 M in-edges, they differ in all four).  AG_TUNE_CACHE names an optional cache file of earlier results. */
 ag_status_t ag_autotune(ag_graph_t g, uint32_t passes, ag_tile_config *best, double *best_pass_us);
 
 /* --------------------------------------------------------------- PageRank */
