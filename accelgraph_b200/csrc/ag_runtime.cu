@@ -241,8 +241,9 @@ static struct
     unsigned char *buf;
     AgControl *ctl;
     cudaEvent_t ev[2];
-    int state; /* 0: not set up, 1: ready, -1: unavailable */
-} g_stage = {nullptr, nullptr, {nullptr, nullptr}, 0};
+    int device; /* of the events: one device's cannot be recorded on another's stream */
+    int state;  /* 0: not set up, 1: ready, -1: unavailable */
+} g_stage = {nullptr, nullptr, {nullptr, nullptr}, -1, 0};
 static std::mutex g_stage_lock;
 
 /* the staging is set up and this thread's until `hold` goes */
@@ -252,18 +253,24 @@ static bool stage_take(std::unique_lock<std::mutex> &hold)
     if (!hold.owns_lock())
         return false;
     if (g_stage.state == 0) {
-        g_stage.state = -1;
         void *p = nullptr;
-        if (cudaHostAlloc(&p, 2 * AG_STAGE_CHUNK + sizeof(AgControl), cudaHostAllocDefault) == cudaSuccess) {
-            if (cudaEventCreateWithFlags(&g_stage.ev[0], cudaEventDisableTiming) == cudaSuccess &&
-                cudaEventCreateWithFlags(&g_stage.ev[1], cudaEventDisableTiming) == cudaSuccess) {
-                g_stage.buf = (unsigned char *)p;
-                g_stage.ctl = (AgControl *)(g_stage.buf + 2 * AG_STAGE_CHUNK);
-                g_stage.state = 1;
-            } else {
-                cudaFreeHost(p);
-            }
+        g_stage.state = -1;
+        if (cudaHostAlloc(&p, 2 * AG_STAGE_CHUNK + sizeof(AgControl), cudaHostAllocPortable) == cudaSuccess) {
+            g_stage.buf = (unsigned char *)p;
+            g_stage.ctl = (AgControl *)(g_stage.buf + 2 * AG_STAGE_CHUNK);
+            g_stage.state = 1;
         }
+        cudaGetLastError();
+    }
+    if (g_stage.state == 1 && g_stage.device != g_ctx.device) {
+        for (cudaEvent_t &e : g_stage.ev) {
+            if (e)
+                cudaEventDestroy(e);
+            e = nullptr;
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+                g_stage.state = -1;
+        }
+        g_stage.device = g_ctx.device;
         cudaGetLastError();
     }
     if (g_stage.state != 1)
