@@ -754,7 +754,8 @@ static ag_status_t plan_device(ag_graph_s *g, uint32_t cap, uint32_t whub)
  * units / bins, FAST and EXACT: 10.8 M in-edges (uniform) 62 / 57 and 63 / 57;
  * 16 M (R-MAT) 63 / 66 and 97 / 72; 17 M (R-MAT, 900 K vertices) 67 / 75 and
  * 87 / 97; 21 M (uniform) 100 / 107 and 100 / 108; 33 M (R-MAT) 98 / 127 and
- * 125 / 148; 65 M (R-MAT) 183 / 265 and 232 / 300. */
+ * 125 / 148; 65 M (R-MAT) 183 / 265 and 232 / 300.  Both limits can be set in
+ * the environment under these names, for an upload to take the other side. */
 #define AG_UNIT_MIN_EDGES 17000000u
 /* Unions above this stay on the pull kernel's loop, one launch per pass: their
  * bins gather from L2 alone.  us per pass, pull kernel / bins, FAST and EXACT:
@@ -821,7 +822,7 @@ static bool want_units(const ag_graph_s *g)
     /* quads are counted in 32 bits: padding is below one quad a row and 32 x
      * AG_UNIT_LONG / 4 a window */
     const uint64_t quads = g->E / 4u + (uint64_t)g->N + ((uint64_t)g->N / AG_UNIT_WIN + 1) * (8 * AG_UNIT_LONG);
-    return !g->ngraphs && g->E >= AG_UNIT_MIN_EDGES && quads < (1ull << 32);
+    return !g->ngraphs && g->N && g->E >= env_u32("AG_UNIT_MIN_EDGES", AG_UNIT_MIN_EDGES) && quads < (1ull << 32);
 }
 
 static ag_status_t plan_unit_rows(ag_graph_s *g, uint32_t *totals)
@@ -1164,7 +1165,8 @@ static ag_status_t upload_impl(const struct GraphCSR *graph, uint32_t flags, con
         UP(cudaMemcpyAsync(g->gstart, gstart_host, (size_t)(ngraphs + 1) * 4, cudaMemcpyHostToDevice, s));
     }
     /* a row partition and a large union run pass by pass on the pull kernel */
-    const bool whole = gather_n == 0 && !(ngraphs && E > AG_UNION_MAX_EDGES), units = whole && want_units(g);
+    const bool whole = gather_n == 0 && !(ngraphs && E > env_u32("AG_UNION_MAX_EDGES", AG_UNION_MAX_EDGES));
+    const bool units = whole && want_units(g);
     uint64_t bin_total = 0;
     uint32_t unit_totals[4] = {0, 0, 0, 0};
     if (units)
