@@ -73,8 +73,7 @@ static inline unsigned ag_sm_grid(unsigned per_sm)
                              whose composers all give their lists away    */
 #endif
 #define AG_XWORDS 64      /* EXACT order: words per hub chunk of integer step
-                             totals (two per 256-value round, the last word
-                             the chunk's data-driven sign tag)              */
+                             totals (two per 256-value round)               */
 #define AG_XROUNDS 31     /* rounds of a chunk with step totals              */
 #define AG_XNOT 0x80000000u /* a round's total that does not apply          */
 #define AG_XFELL 0x100u   /* hub_pred: the chunk had a round summed one value

@@ -61,13 +61,6 @@ __device__ __forceinline__ float ag_ld_cold_f32(const float *p, uint64_t pol)
     return v;
 }
 
-__device__ __forceinline__ uint16_t ag_ld_cold_u16(const uint16_t *p, uint64_t pol)
-{
-    uint16_t v;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
-    return v;
-}
-
 /* per-row data read once per pass: bypass L1 */
 __device__ __forceinline__ uint32_t ag_ld_row_u32(const uint32_t *p)
 {
@@ -82,13 +75,6 @@ __device__ __forceinline__ float ag_ld_rank(const float *p)
 {
     float v;
     asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ uint16_t ag_ld_gather_u16(const uint16_t *p, uint64_t pol)
-{
-    uint16_t v;
-    asm("ld.global.nc.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
     return v;
 }
 

@@ -431,8 +431,8 @@ struct AgPass
     /* whether a hub chunk after the first stages its gathered values, from
      * its record of the pass before (hub_pred): when its starting binade is
      * unknown or it had a round added value by value.  The composing warp
-     * re-gathers an unstaged round if it needs one after all.  SpMV and
-     * 16-bit passes always stage. */
+     * re-gathers an unstaged round if it needs one after all.  A product
+     * always stages. */
     static __device__ __forceinline__ bool hub_staged(uint32_t pr)
     {
         const uint32_t e = pr & 0xffu;

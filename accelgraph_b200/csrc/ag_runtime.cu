@@ -1,15 +1,17 @@
 /*
  * ag_runtime.cu -- device context, graph upload and work planning, the
- * CUDA-graph iteration loop and the status-returning entry points.
+ * launches of solves and products and the status-returning entry points.
  *
  * Replaces the reference's accelerator runtime for this path
  * (02_capi_graph/src/capi_utils/capienv.c: mapGraphCSRToWED :832-874,
  * setupAFUGraphCSR :329-372, startAFU/startCU/waitAFU :375-638,
  * releaseAFU :765-782).  Where the reference crosses the host/accelerator
  * boundary twice per iteration (startCU + waitAFU, pageRank.c:1041-1046),
- * a solve here is one cudaGraphLaunch: init kernel -> WHILE(condition){pull
- * pass} -> normalise, with the condition set on the device by the pass that
- * converged or reached the iteration cap.  Host waits are bounded
+ * a pull solve here is one cooperative launch of the solve kernel (first
+ * contributions, every pass, normalisation), whose grid barrier tells every
+ * CTA that a pass converged or reached the iteration cap.  The integer and
+ * push forms, and unions above AG_UNION_MAX_EDGES, are one cudaGraphLaunch:
+ * init kernel -> WHILE(condition){pass} -> normalise.  Host waits are bounded
  * (AG_WAIT_TIMEOUT_S), after the pattern of the reference's watchdog
  * (accelerator_verification.c:177-320), and return AG_ERR_TIMEOUT instead of
  * exiting.
@@ -235,7 +237,7 @@ extern "C" void ag_rt_host_free(void *ptr, int pinned)
 
 /* Page-locked staging of device-to-host copies: two chunks, and room for a
  * solve's control record.  One copy uses it at a time; a caller that finds it
- * taken copies directly. */
+ * taken waits and copies directly. */
 static struct
 {
     unsigned char *buf;
