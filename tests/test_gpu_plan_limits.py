@@ -138,6 +138,23 @@ def test_hub_rounds_that_leave_their_binade(gpu, oracle, monkeypatch, units):
     dg.release()
 
 
+@pytest.mark.parametrize("name", LENGTHS)
+def test_data_driven_bins(gpu, oracle, name):
+    """Tags of every row class of a bin: the oracle's worklists in EXACT order; and with epsilon 0, when every change is
+    passed on, the plain solve's ranks bit for bit in either order."""
+    ag = gpu
+    g = _graph(ag, LENGTHS[name], len(name))
+    dg = ag.DeviceGraph(g)
+    ref = oracle.pagerank_dd(g.in_edges_idx(), g.in_degree(), g.in_neighbours(), g.out_edges_idx(), g.out_degree(),
+                             g.out_neighbours(), 8, 1e-3)
+    r, res, hist = dg.pagerank(8, 1e-3, order=ag.AG_ORDER_EXACT, data_driven=True, history=8)
+    assert res.iterations == ref["iterations"] and np.array_equal(r, ref["ranks"])
+    assert np.array_equal(hist["active"], ref["active"])
+    for order in (ag.AG_ORDER_FAST, ag.AG_ORDER_EXACT):
+        assert np.array_equal(dg.pagerank(6, 0.0, order=order, data_driven=True)[0], dg.pagerank(6, 0.0, order=order)[0])
+    dg.release()
+
+
 @pytest.mark.parametrize("tiles", [(256, 2048), (64, 128), (32, 32)])
 def test_split_rows_of_the_work_list(gpu, oracle, tiles):
     """A row partition's EXACT passes, split into small chunks: the oracle's ranks bit for bit; and the pull-push form,
