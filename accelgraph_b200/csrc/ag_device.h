@@ -270,6 +270,7 @@ typedef struct AgGraphView
     uint32_t ntasks;
     uint32_t hub_slots;  /* hub chunks in it (slot indexes of HUB items)     */
     uint32_t long_rows;     /* the plan has hub rows */
+    uint32_t max_in_degree;
 } AgGraphView;
 
 /* device planner of the work lists (ag_plan.cu): hub chunks, long rows not

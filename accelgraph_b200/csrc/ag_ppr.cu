@@ -44,7 +44,7 @@
  *
  * More than 32 columns on a graph whose plan has no hub rows run on a kernel
  * without the ring: its code costs the other rows 5 % there (321 against 306
- * at 500 K vertices).
+ * at 500 K vertices).  So do the smallest graphs with rows of some length.
  *
  * The loop stays on the device: after each pass a one-thread kernel counts
  * it and sets a stop flag once no (v, i) pair moved by epsilon; passes that
@@ -69,6 +69,7 @@
                           environment takes sixteen in the kernel without the
                           ring (80 registers, 24 warps): 8.56 against 7.46 ms
                           per pass on ER 2^23, k = 64 */
+#define AG_PPR_WARPS 32u      /* resident warps per SM at that depth         */
 #define AG_PPR_HUB 512u       /* rows with more in-edges go through the ring */
 #define AG_PPR_HUB_SHARE 1024u /* their in-edges per warp that takes them    */
 #define AG_PPR_GROUP 8        /* gathers of one cp.async group             */
@@ -566,7 +567,15 @@ extern "C" ag_status_t ag_ppr_spmm(ag_graph_t g, const uint32_t *sources, uint32
         if (sources[i] >= gv.N)
             return ag_set_error(AG_ERR_INVALID_ARG, "ag_ppr_spmm: source %u >= %u vertices", sources[i], gv.N);
     cudaStream_t s = gv.stream;
-    const uint32_t kp = k > 32 ? AG_PPR_K : (k + 7u) & ~7u;
+    /* Rows that the ring is for, or not.  Without any, a graph of no more rows
+     * than resident warps gives each row a warp whatever k, if some rows are
+     * long: rows that share a warp wait for the longest of them.  us of five
+     * passes, one column, on the shared kernel / so: R-MAT of 1024 vertices
+     * (rows of some hundreds) 203 / 177, 600 137 / 127; uniform 1024 (up to 35)
+     * 91 / 98, 4500 102 / 105. */
+    const bool hub_rows = gv.max_in_degree > AG_PPR_HUB;
+    const bool wide = k > 32 || (!hub_rows && gv.max_in_degree > 64 && gv.N <= ag_sm_grid(AG_PPR_WARPS));
+    const uint32_t kp = wide ? AG_PPR_K : (k + 7u) & ~7u;
     const size_t mat = (size_t)gv.N * kp * sizeof(float);
     float *X = nullptr, *Xn = nullptr, *R = nullptr, *out = nullptr;
     uint32_t *src_dev = nullptr, *hubs = nullptr;
@@ -598,22 +607,25 @@ extern "C" ag_status_t ag_ppr_spmm(ag_graph_t g, const uint32_t *sources, uint32
     PCHK(cudaMallocAsync((void **)&Xn, mat, s));
     PCHK(cudaMallocAsync((void **)&R, mat, s));
     PCHK(cudaMallocAsync((void **)&src_dev, AG_PPR_K * 4, s));
-    PCHK(cudaMallocAsync((void **)&hubs, ((size_t)gv.E / AG_PPR_HUB + 1) * 4, s));
     PCHK(cudaMallocAsync((void **)&ctr, 16, s));
     PCHK(cudaMallocAsync((void **)&state, sizeof(AgPprState), s));
     PCHK(cudaMemsetAsync(ctr, 0, 16, s));
     PCHK(cudaMemsetAsync(state, 0, sizeof(AgPprState), s));
-    if (k <= 16)
-        ppr_pick<8>(&pass_kernel, &init_kernel, &lanes);
-    else if (k <= 32)
-        ppr_pick<16>(&pass_kernel, &init_kernel, &lanes);
-    else
+    if (wide)
         ppr_pick<32>(&pass_kernel, &init_kernel, &lanes);
-    if (k > 32 && !gv.long_rows) {
+    else if (k <= 16)
+        ppr_pick<8>(&pass_kernel, &init_kernel, &lanes);
+    else
+        ppr_pick<16>(&pass_kernel, &init_kernel, &lanes);
+    if (wide && !gv.long_rows) {
         const char *d = getenv("AG_PPR_DEPTH");
         pass_kernel = (d && atoi(d) == 16) ? ag_ppr_wide_kernel<16> : ag_ppr_wide_kernel<AG_PPR_DEPTH>;
         ring = 0;
     }
+    if (!hub_rows)
+        ring = 0;
+    if (ring)
+        PCHK(cudaMallocAsync((void **)&hubs, ((size_t)gv.E / AG_PPR_HUB + 1) * 4, s));
     PCHK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel, AG_PPR_BLK, ring));
     /* init: a few waves; passes: exactly the resident CTAs, so that every
      * warp's share of rows runs at once */

@@ -2421,6 +2421,7 @@ extern "C" ag_status_t ag_rt_graph_view(ag_graph_t g, AgGraphView *v)
     v->ntasks = g->ntasks_fast;
     v->hub_slots = g->nparts;
     v->long_rows = g->bin.nhub || g->unit.nhub;
+    v->max_in_degree = g->max_in_degree;
     return AG_OK;
 }
 
