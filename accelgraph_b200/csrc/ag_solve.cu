@@ -366,14 +366,14 @@ __device__ __forceinline__ uint32_t ag_sv_low_exp(uint32_t pred, uint32_t next)
 
 #define AG_SV_NOT_KEPT 0xffffffffu
 
-/* one round of a hub row value by value (eight consecutive values per lane,
- * lanes below `done` are in s), one lane after another */
-__device__ __forceinline__ float ag_sv_serial(const float *v, float s, uint32_t done)
+/* values of a hub row added one by one (N consecutive ones per lane, lanes
+ * below `done` are in s), one lane after another */
+template <int N> __device__ __forceinline__ float ag_sv_serial(const float *v, float s, uint32_t done)
 {
 #pragma unroll 4
     for (; done < 32u; ++done) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < N; ++i)
             s = __fadd_rn(s, v[i]);
         s = __shfl_sync(0xffffffffu, s, done);
     }
@@ -937,6 +937,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         const uint4 *words = q.hub_words + k0;
         uint16_t *pred = q.hub_pred + k0;
         float s = (float)__ldcg(q.hub_sum + h.z);
+        bool below = false; /* SpMV: the last round added by its values had one below zero */
         uint4 wn = make_uint4(0, 0, 0, 0);
         uint32_t en = 0, em = 0;
         if (lane < rounds) {
@@ -991,6 +992,25 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                     break;
                 /* this round from its values, eight consecutive ones per lane */
                 const uint32_t r = b + out, slot = __shfl_sync(0xffffffffu, w.z, out);
+                if (MODE == AG_MODE_SPMV && below && out < 31u && ((none >> out) & 3u) == 3u) {
+                    /* two such rounds, 16 consecutive values per lane: half
+                     * the hand-overs of s from lane to lane */
+                    const size_t kq = (k0 + r) * (AG_BIN_ROUND / 4) + 4u * lane;
+                    const uint4 *src = reinterpret_cast<const uint4 *>(q.ids) + kq;
+                    const uint32_t j = r * AG_BIN_ROUND + 16u * lane;
+                    if (j + 2u * AG_BIN_ROUND < deg) {
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(src + AG_BIN_ROUND / 2));
+                        if (p.wmode == AG_SPMV_W_GRAPH)
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float4 *>(q.w) + kq +
+                                                                         AG_BIN_ROUND / 2));
+                    }
+                    float v[16];
+                    gather8(__ldg(src), __ldg(src + 1), j, deg, kq, kq + 1, v);
+                    gather8(__ldg(src + 2), __ldg(src + 3), j + 8u, deg, kq + 2, kq + 3, v + 8);
+                    s = ag_sv_serial<16>(v, s, 0u);
+                    done = out + 2u;
+                    continue;
+                }
                 const uint32_t e0 = __shfl_sync(0xffffffffu, lo, out);
                 float v[8];
                 uint32_t from = 0;
@@ -1010,12 +1030,13 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                 } else {
                     const size_t kq = (k0 + r) * (AG_BIN_ROUND / 4) + 2u * lane;
                     const uint4 *src = reinterpret_cast<const uint4 *>(q.ids) + kq;
-                    if (MODE == AG_MODE_SPMV && out < 31u && ((none >> out) & 2u)) {
-                        /* the next round is one of these too */
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(src + AG_BIN_ROUND / 4));
+                    const uint32_t later = out < 31u ? none >> (out + 1u) : 0u;
+                    if (MODE == AG_MODE_SPMV && later) {
+                        /* the next of these rounds */
+                        const uint32_t d = __ffs(later) * (AG_BIN_ROUND / 4);
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(src + d));
                         if (p.wmode == AG_SPMV_W_GRAPH)
-                            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float4 *>(q.w) + kq +
-                                                                         AG_BIN_ROUND / 4));
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float4 *>(q.w) + kq + d));
                     }
                     gather8(__ldg(src), __ldg(src + 1), r * AG_BIN_ROUND + 8u * lane, deg, kq, kq + 1, v);
                     if (MODE == AG_MODE_DD)
@@ -1024,16 +1045,18 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                             v[i] = fabsf(v[i]);
                 }
                 /* SpMV: a value below zero moves M back, so no map holds and the
-                 * round is added value by value.  EXACT, R-MAT of 1 M vertices,
-                 * x centred on 0: 447 us by the three launches, 418 here, the
-                 * largest row's chain; one x in 1000 below zero: 317 and 278 */
+                 * round is added value by value.  us per product, EXACT, weighted
+                 * R-MAT, the three launches / rounds one by one / here, x centred
+                 * on 0: 1 M vertices 443 / 421 / 338, 4 M 1115 / 1217 / 1010; one
+                 * x in 1000 below zero: 283 / 240 / 222, 745 / 857 / 780 */
                 if (MODE == AG_MODE_SPMV) {
                     bool bad = false;
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
                         bad |= !(v[i] >= 0.0f);
-                    if (__any_sync(0xffffffffu, bad)) {
-                        s = ag_sv_serial(v, s, from);
+                    below = __any_sync(0xffffffffu, bad);
+                    if (below) {
+                        s = ag_sv_serial<8>(v, s, from);
                         from = 32u;
                     }
                 }
