@@ -548,9 +548,9 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
         mphase ^= 1u;
     }
 
-    __device__ __forceinline__ float gather(uint32_t u) const
+    template <bool LOW> __device__ __forceinline__ float gather(uint32_t u) const
     {
-        if (low())
+        if (LOW)
             return ag_sv_low<PREC>(u < hot_n ? hot16[u] : ag_sv_ld_u16(c_in16 + u, pol_last, u < p.warm_n));
         return u < hot_n ? hot32[u] : ag_sv_ld_f32(c_in32 + u, pol_last, u < p.warm_n);
     }
@@ -573,7 +573,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     }
 
     /* the group gathers `n` slots (a multiple of 4 is staged) from slot k0 */
-    __device__ __forceinline__ void stage(float *vals, uint64_t k0, uint32_t n) const
+    template <bool LOW> __device__ __forceinline__ void stage(float *vals, uint64_t k0, uint32_t n) const
     {
         const uint4 *i4 = reinterpret_cast<const uint4 *>(q.ids + k0);
         const uint32_t n4 = (n + 3u) >> 2;
@@ -584,14 +584,14 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             if (two)
                 b = ag_ld_stream_u4(i4 + i + AG_SUB_THREADS, pol_first);
             float4 x, y;
-            x.x = gather(a.x);
-            x.y = gather(a.y);
-            x.z = gather(a.z);
-            x.w = gather(a.w);
-            y.x = gather(b.x);
-            y.y = gather(b.y);
-            y.z = gather(b.z);
-            y.w = gather(b.w);
+            x.x = gather<LOW>(a.x);
+            x.y = gather<LOW>(a.y);
+            x.z = gather<LOW>(a.z);
+            x.w = gather<LOW>(a.w);
+            y.x = gather<LOW>(b.x);
+            y.y = gather<LOW>(b.y);
+            y.z = gather<LOW>(b.z);
+            y.w = gather<LOW>(b.w);
             if (MODE == AG_MODE_SPMV) {
                 const float4 wx = weights((k0 >> 2) + i), wy = weights((k0 >> 2) + i + (two ? AG_SUB_THREADS : 0u));
                 times(x, wx);
@@ -658,7 +658,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     }
 
     /* ------------------------------------------------------------ row bin */
-    __device__ __forceinline__ void row_bin(uint32_t k, float *vals)
+    template <bool LOW> __device__ __forceinline__ void row_bin(uint32_t k, float *vals)
     {
         const uint4 ha = __ldg(reinterpret_cast<const uint4 *>(q.bins + k));
         const uint4 hb = __ldg(reinterpret_cast<const uint4 *>(q.bins + k) + 1);
@@ -681,7 +681,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             rp = ag_ld_rank(p.rank + r0 + st);
             od = ag_ld_row_u32(p.outdeg + r0 + st);
         }
-        stage(vals, k0, nslots);
+        stage<LOW>(vals, k0, nslots);
         /* rows without in-edges sum to 0; a hub row is its composer's */
         if (nrows > ha.z + ha.w)
             for (uint32_t i = st; i < nrows; i += AG_SUB_THREADS) {
@@ -832,13 +832,13 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
      * any warps, each at the exponent where the round began in the pass
      * before; a row's first AG_BIN_HEAD values are one lane's chain.  The last
      * chunk of a row to arrive composes the row. */
-    __device__ __forceinline__ void hub_bin(uint32_t k, float *vals)
+    template <bool LOW> __device__ __forceinline__ void hub_bin(uint32_t k, float *vals)
     {
         const uint32_t c0 = k * q.per_bin, nc = min(q.per_bin, q.nhub - c0);
         if (EXACT)
             for (uint32_t i = st; i <= nc * AG_BIN_ROUNDS; i += AG_SUB_THREADS)
                 sh.pred[sub][i] = __ldcg(q.hub_pred + (size_t)c0 * AG_BIN_ROUNDS + i);
-        stage(vals, (uint64_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
+        stage<LOW>(vals, (uint64_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
         ag_sv_sub_sync(sub);
         if (EXACT) {
             for (uint32_t t = sw; t < nc * AG_BIN_ROUNDS; t += AG_SUB_WARPS) {
@@ -902,7 +902,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             __threadfence();
             float s;
             if (EXACT) {
-                s = compose(h);
+                s = compose<LOW>(h);
             } else {
                 double t = 0.0;
                 for (uint32_t c = lane; c < nch; c += 32)
@@ -929,7 +929,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
      * maps); the first that does not apply is added from its values
      * (ag_sv_round), kept by the chunk or gathered again, and the rounds after
      * it go on.  Records where each round began. */
-    __device__ float compose(const uint4 h)
+    template <bool LOW> __device__ float compose(const uint4 h)
     {
         const uint32_t deg = __ldg(p.row_off + h.x + 1) - __ldg(p.row_off + h.x);
         const uint32_t rounds = (deg + AG_BIN_ROUND - 1u) / AG_BIN_ROUND;
@@ -1005,8 +1005,8 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                                                                          AG_BIN_ROUND / 2));
                     }
                     float v[16];
-                    gather8(__ldg(src), __ldg(src + 1), j, deg, kq, kq + 1, v);
-                    gather8(__ldg(src + 2), __ldg(src + 3), j + 8u, deg, kq + 2, kq + 3, v + 8);
+                    gather8<LOW>(__ldg(src), __ldg(src + 1), j, deg, kq, kq + 1, v);
+                    gather8<LOW>(__ldg(src + 2), __ldg(src + 3), j + 8u, deg, kq + 2, kq + 3, v + 8);
                     s = ag_sv_serial<16>(v, s, 0u);
                     done = out + 2u;
                     continue;
@@ -1038,7 +1038,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                         if (p.wmode == AG_SPMV_W_GRAPH)
                             asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const float4 *>(q.w) + kq + d));
                     }
-                    gather8(__ldg(src), __ldg(src + 1), r * AG_BIN_ROUND + 8u * lane, deg, kq, kq + 1, v);
+                    gather8<LOW>(__ldg(src), __ldg(src + 1), r * AG_BIN_ROUND + 8u * lane, deg, kq, kq + 1, v);
                     if (MODE == AG_MODE_DD)
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
@@ -1099,11 +1099,11 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
      * plain sums of the first contributions, so that the first pass composes
      * like the later ones (added value by value it took 2 to 6 ms at R-MAT
      * scale 22 to 24, 6 to 15 later passes).  Two grid barriers. */
-    __device__ __forceinline__ bool predict(float *vals)
+    template <bool LOW> __device__ __forceinline__ bool predict(float *vals)
     {
         for (uint32_t k = blockIdx.x + sub * gridDim.x; k < q.nhb; k += gridDim.x * AG_SUBS) {
             const uint32_t c0 = k * q.per_bin, nc = min(q.per_bin, q.nhub - c0);
-            stage(vals, (uint64_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
+            stage<LOW>(vals, (uint64_t)c0 * AG_BIN_HUB, nc * AG_BIN_HUB);
             ag_sv_sub_sync(sub);
             for (uint32_t t = sw; t < nc * AG_BIN_ROUNDS; t += AG_SUB_WARPS) {
                 const uint4 h = __ldg(q.hubs + c0 + t / AG_BIN_ROUNDS);
@@ -1161,7 +1161,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     /* -------------------------------------------------------------- units */
     /* eight gathered values of a lane's two quads (quads ka and kb of q.ids);
      * those at or past n are -0 (s + -0 = s) */
-    __device__ __forceinline__ void gather8(const uint4 &a, const uint4 &b, uint32_t j, uint32_t n, size_t ka, size_t kb,
+    template <bool LOW> __device__ __forceinline__ void gather8(const uint4 &a, const uint4 &b, uint32_t j, uint32_t n, size_t ka, size_t kb,
                                             float *v) const
     {
         float4 x, y, wx = make_float4(0.0f, 0.0f, 0.0f, 0.0f), wy = wx;
@@ -1171,14 +1171,14 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             if (j + 4u < n)
                 wy = weights(kb);
         }
-        x.x = gather(a.x);
-        x.y = gather(a.y);
-        x.z = gather(a.z);
-        x.w = gather(a.w);
-        y.x = gather(b.x);
-        y.y = gather(b.y);
-        y.z = gather(b.z);
-        y.w = gather(b.w);
+        x.x = gather<LOW>(a.x);
+        x.y = gather<LOW>(a.y);
+        x.z = gather<LOW>(a.z);
+        x.w = gather<LOW>(a.w);
+        y.x = gather<LOW>(b.x);
+        y.y = gather<LOW>(b.y);
+        y.z = gather<LOW>(b.z);
+        y.w = gather<LOW>(b.w);
         if (MODE == AG_MODE_SPMV) {
             times(x, wx);
             times(y, wy);
@@ -1233,7 +1233,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     }
 
     /* the units with the longest rows, one after another */
-    __device__ __forceinline__ void heavy_unit(uint32_t u)
+    template <bool LOW> __device__ __forceinline__ void heavy_unit(uint32_t u)
     {
         const uint32_t b0 = __ldg(q.ubaseq + u), rounds = (__ldg(q.ubaseq + u + 1) - b0) >> 5;
         uint32_t info = 0, od = 0;
@@ -1248,7 +1248,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             if (i + 2 < rounds)
                 pair(b0 + 32u * (i + 2), rounds - i - 2, na, nb);
             float v[8];
-            gather8(a, b, 4u * i, n, unit_quad(b0, i), unit_quad(b0, i + 1), v);
+            gather8<LOW>(a, b, 4u * i, n, unit_quad(b0, i), unit_quad(b0, i + 1), v);
             add8(sum, v, n);
             a = na;
             b = nb;
@@ -1261,7 +1261,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
      * added modulo 2^32).  The next quads (of this unit or the next one) are on their way
      * while a lane's eight gathers travel, and the next batch is drawn one
      * batch ahead. */
-    __device__ __forceinline__ void units(uint32_t bt, uint32_t first_ticket)
+    template <bool LOW> __device__ __forceinline__ void units(uint32_t bt, uint32_t first_ticket)
     {
         if (bt >= q.nbatch)
             return;
@@ -1323,7 +1323,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                     else
                         pair(bn, first_n, na, nb);
                     float v[8];
-                    gather8(a, b, 4u * i, n, unit_quad(b0, i), unit_quad(b0, i + 1), v);
+                    gather8<LOW>(a, b, 4u * i, n, unit_quad(b0, i), unit_quad(b0, i + 1), v);
                     add8(sum, v, n);
                     a = na;
                     b = nb;
@@ -1383,7 +1383,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     }
 
     /* EXACT order: the first AG_BIN_HEAD values of 32 hub rows, one row per lane */
-    __device__ __forceinline__ void heads(uint32_t k)
+    template <bool LOW> __device__ __forceinline__ void heads(uint32_t k)
     {
         const uint32_t i = 32u * k + lane;
         if (i >= q.nhrow)
@@ -1399,7 +1399,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
                 nb = ag_ld_stream_u4(src + j / 4 + 3, pol_first);
             }
             float v[8];
-            gather8(a, b, j, AG_BIN_HEAD, (size_t)first * (AG_BIN_HUB / 4) + j / 4,
+            gather8<LOW>(a, b, j, AG_BIN_HEAD, (size_t)first * (AG_BIN_HUB / 4) + j / 4,
                     (size_t)first * (AG_BIN_HUB / 4) + j / 4 + 1, v);
             add8(sum, v, 0);
             a = na;
@@ -1412,7 +1412,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
 
     /* a hub chunk on one warp, a lane's eight values of a round in registers;
      * FAST: its sum; EXACT: its rounds' maps (predict: their plain sums) */
-    template <bool PREDICT> __device__ __forceinline__ void chunk(uint32_t c)
+    template <bool PREDICT, bool LOW> __device__ __forceinline__ void chunk(uint32_t c)
     {
         const uint4 h = __ldg(q.hubs + c);
         const uint32_t len = (h.w & (AG_BIN_HUB - 1u)) + 1u;
@@ -1443,7 +1443,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             }
             float v[8];
             const size_t kq = (size_t)c * (AG_BIN_HUB / 4) + rd * (AG_BIN_ROUND / 4) + 2u * lane;
-            gather8(a, b, rd * AG_BIN_ROUND + 8u * lane, len, kq, kq + 1, v);
+            gather8<LOW>(a, b, rd * AG_BIN_ROUND + 8u * lane, len, kq, kq + 1, v);
             if (MODE == AG_MODE_DD) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -1492,7 +1492,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     }
 
     /* the hub rows from their chunks, a warp each (a grid barrier before it) */
-    __device__ __forceinline__ void hub_rows()
+    template <bool LOW> __device__ __forceinline__ void hub_rows()
     {
         for (uint32_t i = (tid >> 5) * gridDim.x + blockIdx.x; i < q.nhrow; i += gridDim.x * (AG_SOLVE_BLK / 32)) {
             const uint4 h = __ldg(q.hubs + __ldg(q.hrow + i));
@@ -1511,7 +1511,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             }
             float s;
             if (EXACT) {
-                s = compose(h);
+                s = compose<LOW>(h);
             } else {
                 double t = 0.0;
                 for (uint32_t c = lane; c < nch; c += 32)
@@ -1526,12 +1526,12 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     }
 
     /* every unit and hub chunk of a pass, long chains first */
-    __device__ __forceinline__ bool unit_pass()
+    template <bool LOW> __device__ __forceinline__ bool unit_pass()
     {
         const uint32_t w = (tid >> 5) * gridDim.x + blockIdx.x, nw = gridDim.x * (AG_SOLVE_BLK / 32);
         if (EXACT && iter == 0 && q.nhub) {
             for (uint32_t c = w; c < q.nhub; c += nw)
-                chunk<true>(c);
+                chunk<true, LOW>(c);
             if (!predict_scan())
                 return false;
         }
@@ -1544,19 +1544,50 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             if (lane == 0)
                 ticket = atomicAdd(q.sync + AG_SYNC_BIN, 1u);
             if (t < q.nheavy)
-                heavy_unit(__ldg(q.heavy + t));
+                heavy_unit<LOW>(__ldg(q.heavy + t));
             else if (EXACT && t < q.nheavy + nheads)
-                heads(t - q.nheavy);
+                heads<LOW>(t - q.nheavy);
             else
-                chunk<false>(t - q.nheavy - nheads);
+                chunk<false, LOW>(t - q.nheavy - nheads);
             t = __shfl_sync(0xffffffffu, ticket, 0) + nw;
         }
-        units(t - nlong, nw - nlong);
+        units<LOW>(t - nlong, nw - nlong);
         if (q.nhub) {
             const uint32_t f = flags;
             if (!grid_sync([&] { return f; }))
                 return false;
-            hub_rows();
+            hub_rows<LOW>();
+        }
+        return true;
+    }
+
+    /* every row of a pass; LOW: it gathers 16-bit contributions.  Two bodies:
+     * with the choice at each gather the 16-bit kernels spilled up to 32 bytes.
+     * us per 16-bit pass, FAST / EXACT, chosen at each gather -> here: R-MAT 1 M
+     * vertices 73 / 89 -> 61 / 73, 4 M 240 / 312 -> 170 / 219; uniform 4 M
+     * 168 / 165 -> 152 / 152 */
+    template <bool LOW> __device__ __forceinline__ bool work(float *vals)
+    {
+        if (UNITS)
+            return unit_pass<LOW>();
+        if (EXACT && iter == 0 && q.nhub && !predict<LOW>(vals))
+            return false;
+        const uint32_t nall = q.nhb + q.nbins;
+        uint32_t k = blockIdx.x + sub * gridDim.x;
+        while (k < nall) {
+            /* the next bin's ticket is drawn while this one runs */
+            uint32_t ticket = 0;
+            if (st == 0)
+                ticket = atomicAdd(q.sync + AG_SYNC_BIN, 1u);
+            if (k < q.nhb)
+                hub_bin<LOW>(k, vals);
+            else
+                row_bin<LOW>(k - q.nhb, vals);
+            if (st == 0)
+                sh.next[sub] = ticket + gridDim.x * AG_SUBS;
+            ag_sv_sub_sync(sub);
+            k = sh.next[sub];
+            ag_sv_sub_sync(sub);
         }
         return true;
     }
@@ -1565,31 +1596,9 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     __device__ __forceinline__ bool pass(float *vals)
     {
         start_pass();
-        const uint32_t nall = q.nhb + q.nbins;
-        uint32_t k = blockIdx.x + sub * gridDim.x;
         wait_hot();
-        if (UNITS) {
-            if (!unit_pass())
-                return false;
-        } else if (EXACT && iter == 0 && q.nhub) {
-            if (!predict(vals))
-                return false;
-        }
-        while (!UNITS && k < nall) {
-            /* the next bin's ticket is drawn while this one runs */
-            uint32_t ticket = 0;
-            if (st == 0)
-                ticket = atomicAdd(q.sync + AG_SYNC_BIN, 1u);
-            if (k < q.nhb)
-                hub_bin(k, vals);
-            else
-                row_bin(k - q.nhb, vals);
-            if (st == 0)
-                sh.next[sub] = ticket + gridDim.x * AG_SUBS;
-            ag_sv_sub_sync(sub);
-            k = sh.next[sub];
-            ag_sv_sub_sync(sub);
-        }
+        if (!(PREC != 0 && low() ? work<true>(vals) : work<false>(vals)))
+            return false;
         if (MODE == AG_MODE_SPMV) {
             leave();
             return true;
