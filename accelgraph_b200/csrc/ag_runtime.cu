@@ -1421,7 +1421,10 @@ static ag_status_t solve_ready(ag_graph_s *g)
     const uint32_t w = *g->gave_up;
     if (w == 0)
         return AG_OK;
-    ag_status_t st = solve_recover(g);
+    /* every CTA that gives up writes the word */
+    ag_status_t st = stream_wait(g_ctx.stream, 0);
+    if (st == AG_OK)
+        st = solve_recover(g);
     if (st == AG_OK && w == AG_GAVE_UP_NEW)
         st = ag_set_error(AG_ERR_DEVICE_WAIT, "an earlier solve or product on this graph gave up at a grid barrier; "
                           "it did not finish (nothing was launched now)");

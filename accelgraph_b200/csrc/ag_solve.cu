@@ -380,35 +380,39 @@ template <int N> __device__ __forceinline__ float ag_sv_serial(const float *v, f
     return s;
 }
 
-/* A CTA (one thread) waited in vain for barrier word `gen` to change; it found
- * the arrival word at c when it arrived.  That word decides, once for all
- * CTAs, how a barrier ends: it opens if all have arrived, else it is marked as
- * given up, and whoever arrives later sees the mark.  Returns the barrier word
- * as this CTA has to read it. */
-__device__ __noinline__ uint32_t ag_sv_give_up(uint32_t *sync, uint32_t gen, uint32_t c, uint32_t ctas,
-                                               volatile uint32_t *gave_up)
+/* the arrival word, no CTA there yet, of the barrier after barrier word gen */
+__device__ __forceinline__ uint32_t ag_sv_arrivals(uint32_t gen)
 {
+    return (gen >> AG_GEN_SHIFT) * (AG_COUNT_CTAS + 1u) & ~AG_COUNT_ABORT;
+}
+
+/* One thread of a CTA that waited in vain for barrier word `gen` to change, or
+ * found that another did, and runs nothing more.  The arrival word decides how
+ * the barrier ends: unless all have arrived it is marked as given up, and
+ * nobody opens it any more.  If all have, it opens, and the next one, which
+ * this CTA will not reach, is given up instead.  (Called at the kernel's end:
+ * a call inside the barrier, even of a function of its own, made passes of
+ * FAST bins 1.5 % longer.) */
+__device__ __noinline__ void ag_sv_give_up(uint32_t *sync, uint32_t gen, uint32_t ctas, volatile uint32_t *gave_up)
+{
+    const uint32_t c = ag_sv_arrivals(gen);
     uint32_t now = *((volatile uint32_t *)(sync + AG_SYNC_COUNT));
     bool mine = false;
-    /* this barrier still, not given up, and not all there (at most one round
-     * for each CTA that arrives meanwhile) */
-    while (!mine && (c | now) < AG_COUNT_ABORT && ((now ^ c) & ~AG_COUNT_CTAS) == 0 && (now & AG_COUNT_CTAS) < ctas) {
+    /* (at most one round for each CTA that arrives meanwhile) */
+    while (!mine && now - c < ctas) {
         const uint32_t was = atomicCAS(sync + AG_SYNC_COUNT, now, now | AG_COUNT_ABORT);
         mine = was == now;
         now = was;
     }
-    uint32_t g = gen;
-    if (!mine && c < AG_COUNT_ABORT)
-        /* it opened, or another CTA gave it up: the word follows at once */
+    if (!mine && now < AG_COUNT_ABORT) {
+        uint32_t g = gen;
         for (uint32_t i = 0; g == gen && i < 1u << 20; ++i)
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(g) : "l"(sync + AG_SYNC_GEN) : "memory");
-    if (g == gen) {
-        g = gen | AG_GEN_ABORT;
-        atomicOr(sync + AG_SYNC_GEN, AG_GEN_ABORT);
-        *gave_up = 1u;
-        __threadfence_system();
+        atomicOr(sync + AG_SYNC_COUNT, AG_COUNT_ABORT);
     }
-    return g;
+    atomicOr(sync + AG_SYNC_GEN, AG_GEN_ABORT);
+    *gave_up = 1u;
+    __threadfence_system();
 }
 
 /* ------------------------------------------------------------------ solve */
@@ -452,16 +456,15 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
     /* every CTA's earlier writes are visible to every CTA after it; `close`
      * runs on the last CTA to arrive (all its threads) and returns the flags
      * that the barrier hands on.  The wait is bounded: a CTA that waits in
-     * vain gives the barrier up for all (ag_sv_give_up), and then every CTA,
-     * late ones too, gets false here (or at the kernel's start) and runs
-     * nothing more. */
+     * vain gets false, runs nothing more and gives the barrier up for all
+     * (ag_sv_give_up): every other CTA, late ones too, then gets false here or
+     * at the kernel's start. */
     template <typename F> __device__ __forceinline__ bool grid_sync(F close)
     {
-        uint32_t c = 0;
         __syncthreads();
         if (tid == 0) {
             __threadfence();
-            c = atomicAdd(q.sync + AG_SYNC_COUNT, 1u);
+            const uint32_t c = atomicAdd(q.sync + AG_SYNC_COUNT, 1u);
             sh.last = (c & (AG_COUNT_ABORT | AG_COUNT_CTAS)) == gridDim.x - 1 ? 1u : 0u;
         }
         __syncthreads();
@@ -470,7 +473,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             const uint32_t f = close();
             if (tid == 0) {
                 const uint32_t g = (((gen >> AG_GEN_SHIFT) + 1u) << AG_GEN_SHIFT) | f;
-                q.sync[AG_SYNC_COUNT] = ((c | AG_COUNT_CTAS) + 1u) & ~AG_COUNT_ABORT;
+                q.sync[AG_SYNC_COUNT] = ag_sv_arrivals(g);
                 q.sync[AG_SYNC_BIN] = 0;
                 q.sync[AG_SYNC_KEPT] = 0;
                 sh.gen = g;
@@ -481,9 +484,7 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             uint32_t g = gen;
             for (uint32_t i = 0; g == gen && i < q.spins; ++i)
                 asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(g) : "l"(q.sync + AG_SYNC_GEN) : "memory");
-            if (g == gen)
-                g = ag_sv_give_up(q.sync, gen, c, gridDim.x, q.gave_up);
-            sh.gen = g;
+            sh.gen = g == gen ? gen | AG_GEN_ABORT : g;
             __threadfence();
         }
         __syncthreads();
@@ -1806,17 +1807,16 @@ __global__ void __launch_bounds__(AG_SOLVE_BLK, 1) ag_solve_kernel(const AgSolve
     __shared__ AgSvShared sh;
     AgSolve<MODE, PREC, EXACT, UNITS> s(q, sh);
     float *vals = reinterpret_cast<float *>(ag_sv_dyn + (size_t)q.p.hot_n * 4) + (size_t)s.sub * q.buf;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0)
         ag_sv_mbar_init(&sh.mbar);
-        sh.gen = *((volatile uint32_t *)(q.sync + AG_SYNC_GEN));
-    }
-    /* one answer for the CTA: the word may change now if a barrier is given up */
-    __syncthreads();
-    s.gen = sh.gen;
-    if (s.gen & AG_GEN_ABORT)
-        return;
+    /* a graph that was given up stays so until the host has cleared its words:
+     * the barrier that a solve begins with does not open then; other launches
+     * ask here (all threads together, the mark may be set just now) */
+    s.gen = *((volatile uint32_t *)(q.sync + AG_SYNC_GEN));
     bool ok = true;
     if (MODE == AG_MODE_SPMV) {
+        if (__syncthreads_or(s.gen & AG_GEN_ABORT))
+            return;
         s.iter = 0;
         s.eps = 0.0;
         s.flags = 0;
@@ -1832,29 +1832,31 @@ __global__ void __launch_bounds__(AG_SOLVE_BLK, 1) ag_solve_kernel(const AgSolve
                 q.x_dev[4u * n4 + t0] = __ldg(q.x_in + __ldg(q.p.perm + 4u * n4 + t0));
             ok = s.grid_sync([&] { return 0u; });
         }
-        if (ok)
-            s.pass(vals);
-        return;
-    }
-    if (q.do_init) {
-        s.init(run);
-        const uint32_t f = (run.max_iter > 0 && q.p.N > 0 ? 0u : AG_GEN_STOP) |
-                           (PREC != 0 ? AG_GEN_READ_LOW | AG_GEN_WRITE_LOW : 0u);
-        s.iter = 0;
-        s.eps = run.eps;
-        ok = s.grid_sync([&] { return f; });
+        ok = ok && s.pass(vals);
     } else {
-        volatile AgControl *c = q.p.ctl;
-        s.iter = c->iter;
-        s.eps = c->eps;
-        s.flags = (c->stop ? AG_GEN_STOP : 0u) | (c->mode_read ? AG_GEN_READ_LOW : 0u) |
-                  (c->mode_write ? AG_GEN_WRITE_LOW : 0u);
-        __syncthreads();
+        if (q.do_init) {
+            s.gen &= ~AG_GEN_ABORT;
+            s.init(run);
+            const uint32_t f = (run.max_iter > 0 && q.p.N > 0 ? 0u : AG_GEN_STOP) |
+                               (PREC != 0 ? AG_GEN_READ_LOW | AG_GEN_WRITE_LOW : 0u);
+            s.iter = 0;
+            s.eps = run.eps;
+            ok = s.grid_sync([&] { return f; });
+        } else {
+            ok = !__syncthreads_or(s.gen & AG_GEN_ABORT);
+            volatile AgControl *c = q.p.ctl;
+            s.iter = c->iter;
+            s.eps = c->eps;
+            s.flags = (c->stop ? AG_GEN_STOP : 0u) | (c->mode_read ? AG_GEN_READ_LOW : 0u) |
+                      (c->mode_write ? AG_GEN_WRITE_LOW : 0u);
+        }
+        for (uint32_t n = 0; ok && n < q.max_pass && !(s.flags & AG_GEN_STOP); ++n)
+            ok = s.pass(vals);
+        if (ok && q.do_norm)
+            s.normalise();
     }
-    for (uint32_t n = 0; ok && n < q.max_pass && !(s.flags & AG_GEN_STOP); ++n)
-        ok = s.pass(vals);
-    if (ok && q.do_norm)
-        s.normalise();
+    if (!ok && threadIdx.x == 0)
+        ag_sv_give_up(q.sync, s.gen & ~AG_GEN_ABORT, gridDim.x, q.gave_up);
 }
 
 template <int MODE, int PREC, bool UNITS> static const void *solve_ptr(int exact)

@@ -111,3 +111,28 @@ def test_csr_product_reports(gpu, monkeypatch):
     monkeypatch.delenv("AG_GRID_SPINS")
     assert ag.lib.ag_spmv_pull_ex(C.byref(args), g.ptr, 1, C.byref(out)) == ag.AG_OK
     ag.lib.freeSPMVStats(out)
+
+
+def test_product_behind_a_solve_that_gives_up(gpu, monkeypatch):
+    """A product without a barrier of its own (caller's order, bins) does not run on a graph that was given up."""
+    import ctypes as C
+
+    import torch
+
+    ag = gpu
+    g = _graph(ag, _lengths("bins"), 45)
+    n = g.num_vertices
+    dg = ag.DeviceGraph(g, flags=ag.AG_UPLOAD_KEEP_ORDER)
+    xh = np.random.default_rng(2).random(n, dtype=np.float32)
+    x, y = torch.from_numpy(xh).cuda(), torch.zeros(n, device="cuda")
+    torch.cuda.synchronize()
+    monkeypatch.setenv("AG_GRID_SPINS", "0")
+    dg.launch(6, 1e-6, order=ag.AG_ORDER_EXACT)
+    monkeypatch.delenv("AG_GRID_SPINS")
+    st = ag.lib.ag_spmv_pull_device(dg.h, x.data_ptr(), y.data_ptr(), ag.AG_SPMV_EXACT)
+    if st == ag.AG_OK:  # queued before the host could see it
+        st = ag.lib.ag_synchronize(C.c_double(60.0))
+    assert st == ag.AG_ERR_DEVICE_WAIT and not y.any()
+    want = ag.DeviceGraph(g, flags=ag.AG_UPLOAD_KEEP_ORDER).spmv(xh, ag.AG_SPMV_EXACT)
+    assert np.array_equal(dg.spmv(xh, ag.AG_SPMV_EXACT), want)
+    dg.release()
