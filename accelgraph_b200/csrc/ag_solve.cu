@@ -1815,8 +1815,6 @@ __global__ void __launch_bounds__(AG_SOLVE_BLK, 1) ag_solve_kernel(const AgSolve
     s.gen = *((volatile uint32_t *)(q.sync + AG_SYNC_GEN));
     bool ok = true;
     if (MODE == AG_MODE_SPMV) {
-        if (__syncthreads_or(s.gen & AG_GEN_ABORT))
-            return;
         s.iter = 0;
         s.eps = 0.0;
         s.flags = 0;
@@ -1830,7 +1828,10 @@ __global__ void __launch_bounds__(AG_SOLVE_BLK, 1) ag_solve_kernel(const AgSolve
             }
             if (t0 < (q.p.N & 3u))
                 q.x_dev[4u * n4 + t0] = __ldg(q.x_in + __ldg(q.p.perm + 4u * n4 + t0));
+            s.gen &= ~AG_GEN_ABORT;
             ok = s.grid_sync([&] { return 0u; });
+        } else {
+            ok = !__syncthreads_or(s.gen & AG_GEN_ABORT);
         }
         ok = ok && s.pass(vals);
     } else {
