@@ -484,13 +484,16 @@ template <int MODE, int PREC, bool EXACT, bool UNITS> struct AgSolve
             uint32_t g = gen;
             for (uint32_t i = 0; g == gen && i < q.spins; ++i)
                 asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(g) : "l"(q.sync + AG_SYNC_GEN) : "memory");
-            sh.gen = g == gen ? gen | AG_GEN_ABORT : g;
+            sh.gen = MODE != AG_MODE_MULTI && g == gen ? gen | AG_GEN_ABORT : g;
             __threadfence();
         }
         __syncthreads();
+        /* a wait in vain: the mark in `gen`, in a union the word as it was (either
+         * form in all kernels made unions' or FAST passes 2 to 3 % longer) */
+        const bool stuck = MODE == AG_MODE_MULTI && sh.gen == gen;
         gen = sh.gen;
         flags = gen & 7u;
-        return !(gen & AG_GEN_ABORT);
+        return !stuck && !(gen & AG_GEN_ABORT);
     }
 
     /* the end of a launch without a closing barrier: the last CTA to get here

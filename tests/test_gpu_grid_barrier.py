@@ -136,3 +136,21 @@ def test_product_behind_a_solve_that_gives_up(gpu, monkeypatch):
     want = ag.DeviceGraph(g, flags=ag.AG_UPLOAD_KEEP_ORDER).spmv(xh, ag.AG_SPMV_EXACT)
     assert np.array_equal(dg.spmv(xh, ag.AG_SPMV_EXACT), want)
     dg.release()
+
+
+@pytest.mark.parametrize("order", [0, 1])
+def test_union_gives_up_and_recovers(gpu, monkeypatch, order):
+    ag = gpu
+    mg = ag.MultiGraph([_graph(ag, LENGTHS["hub_rounds"], 46), ag.Graph.rmat(10, 8, seed=3), _graph(ag, [40] * 900, 47)])
+    want, info = mg.pagerank(12, 1e-6, order)
+    for spins in ("0", "0", "50", "500"):
+        monkeypatch.setenv("AG_GRID_SPINS", spins)
+        try:
+            parts, _ = mg.pagerank(12, 1e-6, order)
+            assert spins != "0" and all(np.array_equal(a, b) for a, b in zip(parts, want))
+        except ag.AGError as err:
+            assert err.status == ag.AG_ERR_DEVICE_WAIT
+        monkeypatch.delenv("AG_GRID_SPINS")
+        parts, again = mg.pagerank(12, 1e-6, order)
+        assert all(np.array_equal(a, b) for a, b in zip(parts, want)) and np.array_equal(again["passes"], info["passes"])
+    mg.release()
